@@ -216,7 +216,7 @@ void dgpu_destroy(dgpu_ctx *c) {
   {
     void *ps[] = {c->d_par, c->d_ist, c->d_ann, c->d_cell_ann, c->d_slot_ann, c->d.prim, c->d.cons,
                   c->d.rkcons, c->d.grad, c->d.gradp, c->d.tiph0, c->d.tiph1, c->d.tiphw, c->d.rktiph,
-                  c->d.dphi, c->d.w_ann, c->d.fphi, c->d.frf, c->d.fS, c->d.fdp, c->d.ann_c, c->d.src, c->d.rr, c->d.fstart, c->d.fL, c->d.fR, c->d.fdphi,
+                  c->d.dphi, c->d.w_ann, c->d.frame, c->d.fphi, c->d.frf, c->d.fS, c->d.fdp, c->d.ann_c, c->d.src, c->d.rr, c->d.fstart, c->d.fL, c->d.fR, c->d.fdphi,
                   c->d.fcm, c->d.pair_nf, c->d.pair_jpmin, c->d.pair_T, c->d.pair_seq, c->d.runs,
                   c->d.mdot_part, c->d.counters, c->d.err, c->d.obuf, c->d_stage, c->d_torque,
                   c->d.cfl_ann, c->d.sweep_flag, c->d_zslot_ann, c->d.zfL, c->d.zfR, c->d.zfdphi, c->d.zfcm,
@@ -396,6 +396,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
     c->d.rktiph = (double *)dmalloc(sizeof(double) * N, &ok);
     c->d.dphi = (double *)dmalloc(sizeof(double) * N, &ok);
     c->d.w_ann = (double *)dmalloc(sizeof(double) * A, &ok);
+    c->d.frame = (double *)dmalloc(sizeof(double) * DGPU_FR_N * A, &ok);
     c->d.fphi = (double *)dmalloc(sizeof(double) * NF * N, &ok);
     c->d.frf = (double *)dmalloc(sizeof(double) * NF * (S ? S : 1), &ok);
     c->d.fS = (double *)dmalloc(sizeof(double) * NQ * (S ? S : 1), &ok);

@@ -328,6 +328,7 @@ static int alloc_shadow(struct dgpu_ctx *c, DevPtrs *h, void **mem) {
   SZ(8 * 2 * B);               /* 14: mdot_part */
   SZ(4 * 8);                   /* 15: counters */
   SZ(sizeof(InstState) * (size_t)c->n_inst); /* 16: ist */
+  SZ(8 * DGPU_FR_N * A);       /* 17: frame */
 #undef SZ
   off[0] = 0;
   for (n = 0; n < k; ++n) off[n + 1] = off[n] + sz[n];
@@ -366,6 +367,7 @@ static int alloc_shadow(struct dgpu_ctx *c, DevPtrs *h, void **mem) {
   h->mdot_part = (double *)(m + off[14]);
   h->counters = (unsigned int *)(m + off[15]);
   h->ist = (InstState *)(m + off[16]);
+  h->frame = (double *)(m + off[17]);
   return DGPU_OK;
 }
 

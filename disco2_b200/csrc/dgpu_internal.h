@@ -137,6 +137,13 @@ typedef struct {
 #define DGPU_TUNE_SWEEP 5
 #define DGPU_TUNE_N 6
 
+/* Rows of DevPtrs.frame. */
+#define DGPU_FR_ROM 0    /* sim_rOm_a at the annulus centre */
+#define DGPU_FR_RDROM 1  /* sim_rdrOm_a there */
+#define DGPU_FR_DTOM 2   /* sim_dtOm_a there */
+#define DGPU_FR_FRDROM 3 /* sim_rdrOm_a at the radius of the r-face pair */
+#define DGPU_FR_N 4
+
 /* Device pointers and sizes handed to every kernel. */
 typedef struct {
   int n_inst, n_ann, n_cells, n_slots, n_runs;
@@ -150,6 +157,7 @@ typedef struct {
   double *tiphw;          /* phi edges wrapped into [0, 2pi] (cell_clean_pi) */
   double *rktiph, *dphi;
   double *w_ann;          /* wiph per annulus */
+  double *frame;          /* [DGPU_FR_N][n_ann] frame terms of A_MILOS disks in the substep (k_merge) */
   double *fphi;           /* [8][n_cells] phi-face increments, face (j, j+1) at cell j */
   double *frf;            /* [8][n_slots] r-face increments */
   double *src;            /* [8][n_cells] source increments of the substep (k_source) */

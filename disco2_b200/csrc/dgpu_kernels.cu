@@ -3,8 +3,8 @@
 // One RK substep is eight launches in a CUDA graph:
 //   k_merge    per annulus pair : the r-face list of pair (i, i+1) (face_create
 //                                 / build_jloop) as a checked parallel merge of
-//                                 the two sorted phi-edge lists, and
-//                                 cell_set_w
+//                                 the two sorted phi-edge lists, cell_set_w
+//                                 and the frame terms of a moving frame
 //   k_cellprep per cell         : cell_clean_pi, cell_plm_p, GravMass copy /
 //                                 clean_pi
 //   k_rslope   per r face       : the face slope S and the wrapped offsets of
@@ -225,6 +225,22 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_FACE) k_cellprep(DevPtrs d, Tan
   }
 }
 
+// The frame terms of annulus a that depend on the binary's separation
+// (A_MILOS) into d.frame, one lane each: sim_rOm_a, sim_rdrOm_a and sim_dtOm_a
+// at the annulus centre and sim_rdrOm_a at the radius of pair (i, i+1).
+__device__ __forceinline__ void milos_frame(const DevPtrs &d, const DiskParams &P, const Annulus &A, int a,
+                                            int lane) {
+  if (lane >= DGPU_FR_N) return;
+  const InstState &S = d.ist[A.inst];
+  const double a_sep = S.gr[0] + S.gr[1];
+  const double r = lane == DGPU_FR_FRDROM ? A.f_r : .5 * (A.rp + A.rm);
+  double v;
+  if (lane == DGPU_FR_ROM) v = milos_rom(r, a_sep);
+  else if (lane == DGPU_FR_DTOM) v = milos_dtom(r, a_sep, P.orb_tscale);
+  else v = milos_rdrom(r, a_sep);
+  d.frame[(size_t)lane * d.n_ann + a] = v;
+}
+
 // Per annulus pair (i, i+1) of a disk, one block: the r-face list of
 // face_create/build_jloop (src/Face/face_create_destroy.c:22-193) as a checked
 // parallel merge, and cell_set_w (src/Cell/cell_set_w.c:12-102) of annulus i.
@@ -248,6 +264,7 @@ __device__ __forceinline__ void merge_pair(const DevPtrs &d, int a, int substep)
   const int N = d.n_cells;
   const bool rigid = P.w_numeric == DC_RIGID;
   if (!Z && tid == 0 && !rigid) d.w_ann[a] = A.wnum;
+  if (!Z && tid >= nt - 32 && P.w_analytic == DA_MILOS) milos_frame(d, P, A, a, tid & 31);
   // the pair's arrays: r faces of (a, a+1), or z faces of (a, a+NR)
   int *const pfL = Z ? d.zfL : d.fL, *const pfR = Z ? d.zfR : d.fR;
   double *const pfdphi = Z ? d.zfdphi : d.fdphi, *const pfcm = Z ? d.zfcm : d.fcm;
@@ -776,8 +793,7 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
     v.cm = d.tiphw[cL];
     v.r_cell_L = r;
     v.r_cell_R = r;
-    double a_sep = S.gr[0] + S.gr[1];
-    v.rdr_om = frame_rdrom(P, A.rdrom, r, a_sep);
+    v.rdr_om = frame_val(d, P, A.rdrom, a, DGPU_FR_RDROM);
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
     T Fv[3];
@@ -852,8 +868,7 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
     v.cm = cm;
     v.r_cell_L = r_cell_L;
     v.r_cell_R = r_cell_R;
-    double a_sep = S.gr[0] + S.gr[1];
-    v.rdr_om = frame_rdrom(P, A.f_rdrom, r, a_sep);
+    v.rdr_om = frame_val(d, P, A.f_rdrom, a, DGPU_FR_FRDROM);
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
     T Fv[3];
@@ -1043,10 +1058,9 @@ __device__ __forceinline__ void ann_consts(const DevPtrs &d, int t, const InstSt
   const Annulus &A = d.ann[t];
   const DiskParams &P = d.par[A.inst];
   const double r = 0.5 * (A.rm + A.rp);
-  const double a_sep = S.gr[0] + S.gr[1];
-  const double rom = frame_rom(P, A.rom, r, a_sep);
+  const double rom = frame_val(d, P, A.rom, t, DGPU_FR_ROM);
   const double Omega = rom / r;
-  const double dr_r2Om = 2. * rom + r * frame_rdrom(P, A.rdrom, r, a_sep);
+  const double dr_r2Om = 2. * rom + r * frame_val(d, P, A.rdrom, t, DGPU_FR_RDROM);
   const double kappa2 = 2. * Omega / r * dr_r2Om;
   double kappa = 0.0, ck = 1.0, sk = 0.0;
   if (kappa2 > 0.) {
@@ -1076,7 +1090,6 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
     const int a = d.cell_ann[g];
     const Annulus &A = d.ann[a];
     const DiskParams &P = d.par[A.inst];
-    const double a_sep = S.gr[0] + S.gr[1];
     const double dphi = d.dphi[g];
     const double rm = A.rm, rp = A.rp;
     double phi = d.tiphw[g] - .5 * dphi;
@@ -1104,10 +1117,10 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
         sg.gravdist = R;
       }
     }
-    double w_a = frame_rom(P, A.rom, r, a_sep);
-    sg.rdrOm = frame_rdrom(P, A.rdrom, r, a_sep);
+    double w_a = frame_val(d, P, A.rom, a, DGPU_FR_ROM);
+    sg.rdrOm = frame_val(d, P, A.rdrom, a, DGPU_FR_RDROM);
     sg.Fc = w_a * w_a / r;
-    sg.dtOm = frame_dtom(P, A.dtom, r, a_sep);
+    sg.dtOm = frame_val(d, P, A.dtom, a, DGPU_FR_DTOM);
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
     T gu = 0.0, gpu = 0.0;

@@ -35,6 +35,14 @@ __device__ __forceinline__ void grav_t(GravT<T> &G, const InstState &S, const Di
   }
 }
 
+// Frame terms of annulus a in the substep: A_MILOS's depend on the binary's
+// separation, so they are formed once per annulus and substep (k_merge:
+// milos_frame) instead of by every cell and face -- five pow per term; the
+// other frames' are the host's tables.  k: DGPU_FR_*.
+__device__ __forceinline__ double frame_val(const DevPtrs &d, const DiskParams &P, double tab, int a, int k) {
+  return P.w_analytic == DA_MILOS ? rd(d.frame + (size_t)k * d.n_ann + a) : tab;
+}
+
 // Advanced phi edge of a cell (cell_update_phi, src/Cell/cell_misc.c:59-79).
 __device__ __forceinline__ double new_tiph(double tw, double &rk, double RK, double w_total, double dt, double r,
                                            int *err) {
@@ -64,7 +72,6 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
                                            int substep, int stop, double dt, bool write_rk, T *c) {
   const int N = d.n_cells;
   const DiskParams &P = d.par[A.inst];
-  const InstState &S = d.ist[A.inst];
   const int j = g - A.cell_off;
   const int np = A.np;
   const double RK = substep == 1 ? 0.0 : 0.5;
@@ -212,10 +219,9 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   if (P.has_visc) c[D_TAU] += ldinc<T, NC>(d.src, tp.src, 5, N, g);
   // cell_add_split_fictitious (src/Cell/cell_add_split_fictitious.c:11-44)
   {
-    const double a_sep = S.gr[0] + S.gr[1];
-    const double rom = frame_rom(P, A.rom, r, a_sep);
+    const double rom = frame_val(d, P, A.rom, a, DGPU_FR_ROM);
     const double Omega = rom / r;
-    const double dr_r2Om = 2. * rom + r * frame_rdrom(P, A.rdrom, r, a_sep);
+    const double dr_r2Om = 2. * rom + r * frame_val(d, P, A.rdrom, a, DGPU_FR_RDROM);
     const int NA = d.n_ann;
     const double kappa = NC ? rd(d.ann_c + a) : d.ann_c[a];  // sqrt(kappa2) when kappa2 > 0, else 0
     if (kappa > 0.)
@@ -273,12 +279,10 @@ __device__ __forceinline__ void passive_sum(const DevPtrs &d, const Annulus &A, 
 __device__ __forceinline__ double mesh_advance(const DevPtrs &d, const Annulus &A, int a, int g, int substep,
                                                double dt, double &tn, double &rk) {
   const DiskParams &P = d.par[A.inst];
-  const InstState &S = d.ist[A.inst];
   const double RK = substep == 1 ? 0.0 : 0.5;
   const int j = g - A.cell_off;
   const double r = .5 * (A.rm + A.rp);
-  const double a_sep = S.gr[0] + S.gr[1];
-  const double w_total = rd(d.w_ann + a) + frame_rom(P, A.rom, r, a_sep);
+  const double w_total = rd(d.w_ann + a) + frame_val(d, P, A.rom, a, DGPU_FR_ROM);
   const double *tin = substep == 1 ? d.tiph0 : d.tiph1;
   const int gm1 = j == 0 ? A.cell_off + A.np - 1 : g - 1;
   rk = substep == 1 ? rd(tin + g) : rd(d.rktiph + g);
