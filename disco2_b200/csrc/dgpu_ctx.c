@@ -218,7 +218,7 @@ void dgpu_destroy(dgpu_ctx *c) {
                   c->d.rkcons, c->d.grad, c->d.gradp, c->d.tiph0, c->d.tiph1, c->d.tiphw, c->d.rktiph,
                   c->d.dphi, c->d.w_ann, c->d.frame, c->d.fphi, c->d.frf, c->d.fS, c->d.fdp, c->d.ann_c, c->d.src, c->d.rr, c->d.fstart, c->d.fL, c->d.fR, c->d.fdphi,
                   c->d.fcm, c->d.pair_nf, c->d.pair_jpmin, c->d.pair_T, c->d.pair_seq, c->d.runs,
-                  c->d.mdot_part, c->d.counters, c->d.err, c->d.obuf, c->d_stage, c->d_torque,
+                  c->d.mdot_part, c->d.counters, c->d.err, c->d.obuf, c->d_ob_cell, c->d_stage, c->d_torque,
                   c->d.cfl_ann, c->d.sweep_flag, c->d_zslot_ann, c->d.zfL, c->d.zfR, c->d.zfdphi, c->d.zfcm,
                   c->d.zfstart, c->d.zrr, c->d.zruns, c->d.zpair_nf, c->d.zpair_jpmin, c->d.zpair_T,
                   c->d.zpair_seq, c->d.zfS, c->d.zfdp, c->d.zfrf, c->d.gradz};
@@ -335,9 +335,6 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   c->d.n_zslots = zslots;
   c->d.n_zruns = zruns;
   c->d.has_z = has_z;
-  c->d.max_nz = 1;
-  for (k = 0; k < n; ++k)
-    if (c->sims[k]->NZ > c->d.max_nz) c->d.max_nz = c->sims[k]->NZ;
   /* one 3-D disk: its ghost layers are the first and last cells, and the
    * periodic z copy launches over those alone */
   c->d.zghost = 0;
@@ -438,7 +435,10 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
       c->d.gradz = (double *)dmalloc(sizeof(double) * 5 * N, &ok);
     }
     c->d.err = (int *)dmalloc(sizeof(int), &ok);
-    if (n_ob > 0) c->d.obuf = (double *)dmalloc(sizeof(double) * NQ * (size_t)n_ob, &ok);
+    if (n_ob > 0) {
+      c->d.obuf = (double *)dmalloc(sizeof(double) * NQ * (size_t)n_ob, &ok);
+      c->d_ob_cell = (int *)dmalloc(sizeof(int) * (size_t)n_ob, &ok);
+    }
     c->d_stage = (double *)dmalloc(sizeof(double) * NQ * (size_t)maxcells, &ok);
     c->d_torque = (double *)dmalloc(sizeof(double) * ((size_t)maxcells / dgk_block_size() + 8), &ok);
   }
@@ -495,6 +495,10 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   c->d.ann = c->d_ann;
   c->d.cell_ann = c->d_cell_ann;
   c->d.slot_ann = c->d_slot_ann;
+  c->d.ob_cell = c->d_ob_cell;
+  c->d.ob_three = 0;
+  for (k = 0; k < n; ++k)
+    if ((c->h_par[k].outflow & 1) && c->h_par[k].NR == 3) c->d.ob_three = 1;
   c->d.zslot_ann = c->d_zslot_ann;
   if (cudaMemcpy(c->d_par, c->h_par, sizeof(DiskParams) * (size_t)n, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(c->d_ann, c->h_ann, sizeof(Annulus) * (size_t)c->n_ann, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -512,6 +516,23 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   free(h_cell_ann);
   free(h_slot_ann);
   free(h_zslot_ann);
+  if (n_ob > 0) {
+    /* the cells of the outflow boundary's columns: the annuli with an ob_off,
+     * in the order the offsets were given out */
+    int *h = (int *)malloc(sizeof(int) * (size_t)n_ob), bad = !h;
+    if (h) {
+      int a, j;
+      for (a = 0; a < c->n_ann; ++a)
+        for (j = 0; c->h_ann[a].ob_off >= 0 && j < c->h_ann[a].np; ++j)
+          h[c->h_ann[a].ob_off + j] = c->h_ann[a].cell_off + j;
+      bad = cudaMemcpy(c->d_ob_cell, h, sizeof(int) * (size_t)n_ob, cudaMemcpyHostToDevice) != cudaSuccess;
+      free(h);
+    }
+    if (bad) {
+      dgpu_destroy(c);
+      return fail(NULL, DGPU_ERR_CUDA, "table upload failed");
+    }
+  }
   *out = c;
   return DGPU_OK;
 }

@@ -181,6 +181,8 @@ typedef struct {
   double *obuf;           /* [5 + n_pass][n_ob] prims, before damping, of the annuli the outflow
                              boundary reads or writes (k_update writes them, k_outflow finishes them) */
   int n_ob;
+  const int *ob_cell;     /* [n_ob] cell of each obuf column */
+  int ob_three;           /* some disk with an outflow boundary has three annuli */
   int n_pass;             /* passive-scalar planes (largest NUM_N of the disks): prim, cons, rkcons,
                              grad and gradp hold 5 + n_pass planes, fS 5 + n_pass, fphi and frf
                              8 + n_pass (the passive increments after the viscous ones) */
@@ -191,7 +193,6 @@ typedef struct {
   /* z faces of 3-D disks (NZ > 1): the same structures as the r faces, per
      z pair (ring a, ring a+NR) of each ring a with k < NZ-1 */
   int n_zslots, n_zruns, has_z;
-  int max_nz;             /* largest NZ of the disks */
   const int *zslot_ann;   /* z-face slot -> ring of its pair (the lower ring) */
   int *zfL, *zfR;         /* z-face cells (global); zfL = -1 past the list of a pair */
   double *zfdphi, *zfcm;
@@ -263,7 +264,7 @@ int dgk_flux_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
 int dgk_update(const DevPtrs *d, const TanPtrs *t, int substep, int stop, void *stream);
 int dgk_update_stage(const DevPtrs *d, int substep, int stop, void *stream);
 /* the outflow radial boundary, its damping and cell_calc_cons on the annuli
- * it rewrites (one block per disk); after k_update, for stop >= 6 */
+ * it rewrites (one thread per boundary cell); after k_update, for stop >= 6 */
 int dgk_outflow(const DevPtrs *d, int stop, void *stream);
 /* 3-D disks: the z-face list (zmerge), z-face slopes, z slopes (cell_plm_rz
  * with Z_DIR), z-face fluxes, and the single-rank periodic z copy of

@@ -24,7 +24,7 @@
 //                                 fixed radial boundary, cell_bc_damp and
 //                                 cell_calc_cons; its last block advances the
 //                                 GravMass state
-// and, for disks with the outflow radial boundary, k_outflow per disk
+// and, for disks with the outflow radial boundary, k_outflow per boundary cell
 // (cell_boundary_outflow_r).  k_merge runs beside k_cellprep on a second
 // stream, and k_source then k_flux_phi beside k_flux_r.
 //
@@ -1649,88 +1649,168 @@ __global__ void __launch_bounds__(BLK) k_calc_cons(DevPtrs d, TanPtrs tp) {
   for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q) d.cons[(size_t)q * N + g] = ld(d.prim, q, N, g) * val(c[D_DDD]);
 }
 
-// One pass of cell_boundary_outflow_r (src/Cell/cell_boundary.c:14-139) over
-// the r faces of annulus pair (i, i+1) of the substep's face list: every cell
-// of the rewritten annulus (i when outer == 0, else i+1) takes the sum, in face
-// order, of prim * dA of the cells across its faces, divided by
-// dz * FacePos(i) * dphi.  The reference's build constants EXTRAP_BC, SS_BCS,
-// diode and KEP_BNDRY are 0 (header.h); its inner term
-// (prim - 0 * grad * (...) / 2.) * dA is prim * dA for a finite slope.  A cell
-// with no face keeps its own value, divided (the reference zeroes only the
+// cell_boundary_outflow_r (src/Cell/cell_boundary.c:14-139) runs three passes
+// over the substep's r faces, each reading the one before: annulus 0 from
+// annulus 1 (unless NoInnerBC == 1), NR-2 from NR-3, NR-1 from the new NR-2.
+// A pass gives every cell the sum, in face order, of prim * dA of the cells
+// across its faces, divided by dz * FacePos(i) * dphi.  The reference's build
+// constants EXTRAP_BC, SS_BCS, diode and KEP_BNDRY are 0 (header.h); its inner
+// term (prim - 0 * grad * (...) / 2.) * dA is prim * dA for a finite slope.  A
+// cell with no face keeps its own value, divided (the reference zeroes only the
 // cells its face loop visits).
-__device__ __forceinline__ void outflow_pass(const DevPtrs &d, const DiskParams &P, int base, int i, int outer) {
-  const int a = base + i + outer;
+//
+// Every pass is formed here from the prims k_update left in obuf, which nothing
+// writes any more: a cell of NR-1 forms the two or three NR-2 values it reads
+// again itself.  So the passes need no barrier, and the work is spread over
+// the chip: OB_LANES lanes per boundary cell, a face each, whose terms are
+// added in face order by shuffles.  It is a chain of dependent loads (ranges,
+// face, cell) that bounds this kernel, not its few thousand cells.
+#define OB_LANES 8
+
+// The value of cell g of annulus a after its pass, formed by one thread from
+// the prims of the annulus read, four faces' loads in flight at a time.  PASS
+// 1: annulus 0 from 1; 2: NR-2 from NR-3.  NQ: 5, or 5 + DGPU_MAX_PASSIVE
+// (planes past nq are skipped).
+template <int PASS, int NQ>
+__device__ __forceinline__ void outflow_value(const DevPtrs &d, const DiskParams &P, int a, int g, int nq,
+                                              double *v) {
   const Annulus &A = d.ann[a];
-  const Annulus &S = d.ann[base + i + 1 - outer];  // the annulus read
-  const double rf = d.ann[base + i].f_r;           // FacePos(i)
+  constexpr int outer = PASS != 1;
+  const Annulus &Q = d.ann[a - outer];              // the pair (i, i+1) walked
+  const Annulus &S = d.ann[outer ? a - 1 : a + 1];  // the annulus read
   const size_t NB = d.n_ob;
-  const int nq = 5 + P.num_n;
-  const int np = nq - 5;
-  for (int j = threadIdx.x; j < A.np; j += blockDim.x) {
-    const int g = A.cell_off + j;
-    // the five hydro sums in registers, the passive scalars' apart
-    double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, sp[DGPU_MAX_PASSIVE];
-    for (int k = 0; k < np; ++k) sp[k] = 0.0;
-    int nface = 0;
-    for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int, int side) {
-      if (side != outer) return;
-      const int o = S.ob_off + ((outer ? F.cL : F.cR) - S.cell_off);
-      const double dA = F.r * F.dphi * F.dperp;
+  const int off = S.ob_off - S.cell_off;
+  const double fr = Q.f_r, fperp = Q.f_dperp;
+  double s[NQ];
 #pragma unroll
-      for (int q = 0; q < 5; ++q) s[q] += d.obuf[q * NB + o] * dA;
-      for (int k = 0; k < np; ++k) sp[k] += d.obuf[(5 + k) * NB + o] * dA;
-      ++nface;
-    });
-    const double dA = A.dz * rf * d.dphi[g];
-    const size_t self = (size_t)A.ob_off + j;
+  for (int q = 0; q < NQ; ++q) s[q] = 0.0;
+  int nface = 0;
+  for_cell_rface_ranges(d, A, a, g, P.NR, [&](int n0, int n1, int side) {
+    if (side != outer) return;
+    for (int n = n0; n < n1; n += 4) {
+      int c[4];
+      double dA[4];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) d.obuf[q * NB + self] = (nface ? s[q] : d.obuf[q * NB + self]) / dA;
-    for (int k = 0; k < np; ++k)
-      d.obuf[(5 + k) * NB + self] = (nface ? sp[k] : d.obuf[(5 + k) * NB + self]) / dA;
-  }
+      for (int k = 0; k < 4; ++k) {
+        const int f = min(n + k, n1 - 1);
+        c[k] = off + rd((outer ? d.fL : d.fR) + f);
+        dA[k] = fr * rd(d.fdphi + f) * fperp;
+      }
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        if (NQ > 5 && q >= nq) break;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double u = rd(d.obuf + q * NB + c[k]);
+          if (n + k < n1) s[q] += u * dA[k];
+        }
+      }
+      nface += min(4, n1 - n);
+    }
+  });
+  const double dA = A.dz * fr * d.dphi[g];
+  const size_t self = (size_t)A.ob_off + (g - A.cell_off);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q)
+    if (NQ == 5 || q < nq) v[q] = (nface ? s[q] : rd(d.obuf + q * NB + self)) / dA;
 }
 
-// The outflow radial boundary of one layer of a disk per block (blockIdx.x:
-// the disk, blockIdx.y: the layer), in the reference's order: annulus 0 from
-// annulus 1 (unless NoInnerBC == 1), NR-2 from NR-3, NR-1 from the new NR-2;
-// each pass reads the previous one's results.  The r faces join rings of one
-// layer, so the layers are independent.  Then the rewritten annuli get
-// cell_bc_damp and, for stop 7, cell_calc_cons.
-__global__ void __launch_bounds__(BLK) k_outflow(DevPtrs d, int stop) {
-  const DiskParams &P = d.par[blockIdx.x];
-  if (!(P.outflow & 1) || (int)blockIdx.y >= P.NZ) return;
-  const int NR = P.NR, N = d.n_cells;
-  const int base = P.ann_base + (int)blockIdx.y * NR;
+// The outflow radial boundary, OB_LANES threads per cell of the annuli it
+// reads or writes (ob_cell): the value after the cell's pass, then, for the
+// rewritten annuli, cell_bc_damp and, for stop 7, cell_calc_cons.  PS: some
+// disk carries passive scalars.  THREE: some disk has three annuli, where NR-2
+// is annulus 1 and reads the new annulus 0.
+#define OUTFLOW_BLK 64
+template <bool PS, bool THREE>
+__global__ void __launch_bounds__(OUTFLOW_BLK) k_outflow(DevPtrs d, int stop) {
+  constexpr int NQ = PS ? 5 + DGPU_MAX_PASSIVE : 5;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) / OB_LANES;
+  const int lane = threadIdx.x & 31, sub = lane % OB_LANES, first = lane - sub;
+  const unsigned group = ((1u << OB_LANES) - 1u) << first;
+  if (t >= d.n_ob) return;
+  const int g = rd(d.ob_cell + t), N = d.n_cells;
+  const int a = rd(d.cell_ann + g);
+  const Annulus &A = d.ann[a];
+  if (!(A.kind & DGPU_AK_OUT_DST)) return;
+  const DiskParams &P = d.par[A.inst];
   const size_t NB = d.n_ob;
-  if (P.outflow & 2) outflow_pass(d, P, base, 0, 0);
-  __syncthreads();
-  outflow_pass(d, P, base, NR - 3, 1);
-  __syncthreads();
-  outflow_pass(d, P, base, NR - 2, 1);
-  __syncthreads();
-  for (int k = 0; k < 3; ++k) {
-    const int i = k == 0 ? 0 : NR - 3 + k;
-    const int a = base + i;
-    const Annulus &A = d.ann[a];
-    if (!(A.kind & DGPU_AK_OUT_DST)) continue;
-    const double r = .5 * (A.rm + A.rp);
-    for (int j = threadIdx.x; j < A.np; j += blockDim.x) {
-      const int g = A.cell_off + j;
-      double pr[5], c[5];
+  const int nq = PS ? 5 + P.num_n : 5;
+  const int pass = A.i == P.NR - 1 ? 3 : A.i == P.NR - 2 ? 2 : 1;
+  const bool chain1 = THREE && P.NR == 3 && (P.outflow & 2);
+  const int outer = pass != 1;
+  const Annulus &Q = d.ann[a - outer];
+  const Annulus &S = d.ann[outer ? a - 1 : a + 1];
+  double s[NQ];
 #pragma unroll
-      for (int q = 0; q < 5; ++q) pr[q] = d.obuf[q * NB + A.ob_off + j];
-      bc_damp(d, A, a, pr);
+  for (int q = 0; q < NQ; ++q) s[q] = 0.0;
+  int nface = 0;
+  for_cell_rface_ranges(d, A, a, g, P.NR, [&](int n0, int n1, int side) {
+    if (side != outer) return;
+    for (int n = n0; n < n1; n += OB_LANES) {
+      const int nk = min(OB_LANES, n1 - n);
+      double u[NQ], dA = 0.0;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) d.prim[(size_t)q * N + g] = pr[q];
-      for (int q = 5; q < 5 + P.num_n; ++q) d.prim[(size_t)q * N + g] = d.obuf[q * NB + A.ob_off + j];
-      if (stop >= 7) {
-        const double dV = A.dv_half * d.dphi[g] * A.dz;
-        prim2cons(pr, c, r, dV, P.gamma);
+      for (int q = 0; q < NQ; ++q) u[q] = 0.0;
+      if (sub < nk) {
+        const int f = n + sub;
+        const int c = rd((outer ? d.fL : d.fR) + f);
+        dA = Q.f_r * rd(d.fdphi + f) * Q.f_dperp;
+        if (THREE && pass == 3 && chain1) {
+          const Annulus &S1 = d.ann[a - 1], &Q1 = d.ann[a - 2];
+          int nf1 = 0;
+          for_cell_rface_ranges(d, S1, a - 1, c, P.NR, [&](int m0, int m1, int side1) {
+            if (side1 != 1) return;
+            for (int m = m0; m < m1; ++m) {
+              double v[NQ];
+              outflow_value<1, NQ>(d, P, a - 2, rd(d.fL + m), nq, v);
+              const double dA1 = Q1.f_r * rd(d.fdphi + m) * Q1.f_dperp;
+              for (int q = 0; q < nq; ++q) u[q] += v[q] * dA1;
+              ++nf1;
+            }
+          });
+          const double dA1 = S1.dz * Q1.f_r * d.dphi[c];
+          for (int q = 0; q < nq; ++q)
+            u[q] = (nf1 ? u[q] : rd(d.obuf + q * NB + (S1.ob_off + (c - S1.cell_off)))) / dA1;
+        } else if (pass == 3) {
+          outflow_value<2, NQ>(d, P, a - 1, c, nq, u);
+        } else if (THREE && pass == 2 && chain1) {
+          outflow_value<1, NQ>(d, P, a - 1, c, nq, u);
+        } else {
 #pragma unroll
-        for (int q = 0; q < 5; ++q) d.cons[(size_t)q * N + g] = c[q];
-        for (int q = 5; q < 5 + P.num_n; ++q) d.cons[(size_t)q * N + g] = d.obuf[q * NB + A.ob_off + j] * c[D_DDD];
+          for (int q = 0; q < NQ; ++q)
+            if (!PS || q < nq) u[q] = rd(d.obuf + q * NB + (S.ob_off + (c - S.cell_off)));
+        }
       }
+      // the terms of these faces in face order
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) u[q] *= dA;
+      for (int k = 0; k < nk; ++k)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) s[q] += __shfl_sync(group, u[q], first + k);
+      nface += nk;
     }
+  });
+  if (sub != 0) return;
+  const double dphi = d.dphi[g];
+  const double dA = A.dz * Q.f_r * dphi;
+  const size_t self = (size_t)A.ob_off + (g - A.cell_off);
+  double pr[NQ], c[5];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q)
+    if (!PS || q < nq) pr[q] = (nface ? s[q] : rd(d.obuf + q * NB + self)) / dA;
+  bc_damp(d, A, a, pr);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q)
+    if (!PS || q < nq) d.prim[(size_t)q * N + g] = pr[q];
+  if (stop >= 7) {
+    const double r = .5 * (A.rm + A.rp);
+    const double dV = A.dv_half * dphi * A.dz;
+    prim2cons(pr, c, r, dV, P.gamma);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) d.cons[(size_t)q * N + g] = c[q];
+#pragma unroll
+    for (int q = 5; q < NQ; ++q)
+      if (q < nq) d.cons[(size_t)q * N + g] = pr[q] * c[D_DDD];
   }
 }
 
@@ -1952,7 +2032,11 @@ int dgk_sweep(const DevPtrs *d, int substep, void *stream) {
 }
 int dgk_outflow(const DevPtrs *d, int stop, void *stream) {
   if (d->n_ob <= 0 || stop < 6) return 0;
-  k_outflow<<<dim3(d->n_inst, d->max_nz), BLK, 0, (cudaStream_t)stream>>>(*d, stop);
+  const int grid = (int)(((long long)d->n_ob * OB_LANES + OUTFLOW_BLK - 1) / OUTFLOW_BLK);
+  cudaStream_t s_ = (cudaStream_t)stream;
+  if (d->n_pass > 0) k_outflow<true, true><<<grid, OUTFLOW_BLK, 0, s_>>>(*d, stop);
+  else if (d->ob_three) k_outflow<false, true><<<grid, OUTFLOW_BLK, 0, s_>>>(*d, stop);
+  else k_outflow<false, false><<<grid, OUTFLOW_BLK, 0, s_>>>(*d, stop);
   return (int)cudaGetLastError();
 }
 int dgk_calc_cons(const DevPtrs *d, const TanPtrs *t, void *stream) {
