@@ -227,7 +227,8 @@ void dgpu_destroy(dgpu_ctx *c) {
   }
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   if (c->side) cudaStreamDestroy(c->side);
-  for (k = 0; k < 4; ++k)
+  if (c->side2) cudaStreamDestroy(c->side2);
+  for (k = 0; k < DCTX_FORKS; ++k)
     if (c->fork[k]) cudaEventDestroy(c->fork[k]);
   if (c->sims) {
     for (k = 0; k < c->n_inst; ++k) dsim_free(c->sims[k]);
@@ -237,6 +238,10 @@ void dgpu_destroy(dgpu_ctx *c) {
   free(c->h_ann);
   free(c);
 }
+
+/* A context whose cell kernels run in at most two waves of blocks (148 SMs x
+ * 4 blocks x 256 cells): its launches are bound by latency. */
+static int few_waves(const struct dgpu_ctx *c) { return c->n_cells <= 2 * 148 * 4 * 256; }
 
 int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dgpu_ctx **out) {
   struct dgpu_ctx *c;
@@ -362,8 +367,9 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
     c->own_stream = 1;
   }
   {
-    int k, bad = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess;
-    for (k = 0; k < 4 && !bad; ++k)
+    int k, bad = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+                 cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking) != cudaSuccess;
+    for (k = 0; k < DCTX_FORKS && !bad; ++k)
       bad = cudaEventCreateWithFlags(&c->fork[k], cudaEventDisableTiming) != cudaSuccess;
     if (bad) {
       free(h_cell_ann);
@@ -483,6 +489,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   for (k = 0; k < n; ++k)
     if (c->h_par[k].rho_sink_on == 1) c->fused_ok = 0;
   c->fused = 0;
+  c->d.form_dt = few_waves(c);
   c->d.n_inst = n;
   c->d.n_ann = c->n_ann;
   c->d.n_cells = c->n_cells;
@@ -760,9 +767,14 @@ int dgpu_init_state(dgpu_ctx *c, int inst) {
   return rc;
 }
 
-int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub, int mode, double *rec, const int *rec_idx) {
-  /* the layout of the step graph: merge beside cellprep, source and the phi
-   * faces beside the r faces */
+int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub) {
+  /* merge beside cellprep; the sources and the phi faces beside the r faces.
+   * Up to two waves of cell blocks a launch is little longer than one thread's instruction stream, so the phi
+   * faces take a stream of their own (128 us a step for the 59,746-cell disk
+   * against 136 behind the sources, 357 against 366 for 258,078 cells); on
+   * larger contexts three kernels at once only share the SMs (the 12-disk
+   * sweep 392 against 388 ms for 80 steps) */
+  cudaStream_t phi = few_waves(c) ? c->side2 : c->side;
   CK(cudaEventRecord(c->fork[0], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[0], 0));
   CKK(dgk_merge(&c->d, sub, c->side));
@@ -771,19 +783,20 @@ int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub, int mode, double
   CK(cudaStreamWaitEvent(c->stream, c->fork[1], 0));
   CKK(dgk_rslope(&c->d, t, c->stream));
   CKK(dgk_plm_r(&c->d, t, sub, c->stream));
-  if (mode == DCTX_ADJPREP) {
-    CKK(dgk_ann_consts(&c->d, sub, c->stream));
-    return DGPU_OK;
-  }
+  if (sub == 1 && !c->d.form_dt) CKK(dgk_dt(&c->d, c->stream));
   CK(cudaEventRecord(c->fork[2], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[2], 0));
+  if (phi != c->side) CK(cudaStreamWaitEvent(phi, c->fork[2], 0));
   CKK(dgk_source(&c->d, t, sub, c->side));
-  CKK(dgk_flux_phi(&c->d, t, sub, c->side));
+  CKK(dgk_flux_phi(&c->d, t, sub, phi));
   CKK(dgk_flux_r(&c->d, t, sub, c->stream));
   CK(cudaEventRecord(c->fork[3], c->side));
   CK(cudaStreamWaitEvent(c->stream, c->fork[3], 0));
-  if (mode == DCTX_REC) CKK(dgk_update_rec(&c->d, sub, rec, rec_idx, c->stream));
-  else CKK(dgk_update(&c->d, t, sub, 7, c->stream));
+  if (phi != c->side) {
+    CK(cudaEventRecord(c->fork[4], phi));
+    CK(cudaStreamWaitEvent(c->stream, c->fork[4], 0));
+  }
+  CKK(dgk_update(&c->d, t, sub, 7, c->stream));
   if (c->n_ob > 0) CKK(dgk_outflow(&c->d, 7, c->stream));
   return DGPU_OK;
 }
@@ -809,6 +822,7 @@ static int launch_substep_3d(struct dgpu_ctx *c, int sub) {
   CKK(dgk_plm_z(&c->d, c->side));
   CKK(dgk_rslope(&c->d, NULL, c->stream));
   CKK(dgk_plm_r(&c->d, NULL, sub, c->stream));
+  if (sub == 1 && !c->d.form_dt) CKK(dgk_dt(&c->d, c->stream));
   CK(cudaEventRecord(c->fork[3], c->side));
   CK(cudaStreamWaitEvent(c->stream, c->fork[3], 0));
   CK(cudaEventRecord(c->fork[0], c->stream));
@@ -843,25 +857,8 @@ int dctx_launch_step(struct dgpu_ctx *c) {
     return DGPU_OK;
   }
   for (sub = 1; sub <= 2; ++sub) {
-    /* k_merge (per annulus pair) alongside k_cellprep (per cell) */
-    CK(cudaEventRecord(c->fork[0], c->stream));
-    CK(cudaStreamWaitEvent(c->side, c->fork[0], 0));
-    CKK(dgk_merge(&c->d, sub, c->side));
-    CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
-    CK(cudaEventRecord(c->fork[1], c->side));
-    CK(cudaStreamWaitEvent(c->stream, c->fork[1], 0));
-    CKK(dgk_rslope(&c->d, NULL, c->stream));
-    CKK(dgk_plm_r(&c->d, NULL, sub, c->stream));
-    /* k_source and the phi faces (per cell) alongside the r faces (per face) */
-    CK(cudaEventRecord(c->fork[2], c->stream));
-    CK(cudaStreamWaitEvent(c->side, c->fork[2], 0));
-    CKK(dgk_source(&c->d, NULL, sub, c->side));
-    CKK(dgk_flux_phi(&c->d, NULL, sub, c->side));
-    CKK(dgk_flux_r(&c->d, NULL, sub, c->stream));
-    CK(cudaEventRecord(c->fork[3], c->side));
-    CK(cudaStreamWaitEvent(c->stream, c->fork[3], 0));
-    CKK(dgk_update(&c->d, NULL, sub, 7, c->stream));
-    if (c->n_ob > 0) CKK(dgk_outflow(&c->d, 7, c->stream));
+    int rc = dctx_substep(c, NULL, sub);
+    if (rc) return rc;
   }
   return DGPU_OK;
 }
@@ -945,6 +942,7 @@ int dgpu_step_rk2_timed(dgpu_ctx *c, int nsteps, double *kernel_ms) {
       CKK(dgk_rslope(&c->d, NULL, c->stream));
       CK(cudaEventRecord(ev[e++], c->stream));
       CKK(dgk_plm_r(&c->d, NULL, sub, c->stream));
+      if (sub == 1 && !c->d.form_dt) CKK(dgk_dt(&c->d, c->stream));
       /* 3-D: the z faces, whose slopes the viscous source reads, in the
        * plm_r slot (no-ops for 2-D disks) */
       CKK(dgk_zslope(&c->d, c->stream));
@@ -1061,14 +1059,16 @@ int dgpu_stage(dgpu_ctx *c, int phase) {
   /* phases 8-15: the whole first substep (its k_update also moves the
    * GravMass, as timestep_rk2 does between the substeps), then the second */
   if (sub == 2) {
-    int rc = dctx_substep(c, NULL, 1, DCTX_FULL, NULL, NULL);
+    int rc = dctx_substep(c, NULL, 1);
     if (rc) return rc;
   }
   CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
   CKK(dgk_merge(&c->d, sub, c->stream));
-  /* the CFL minimum (and dt) come from k_plm_r; PLM results are kept only from phase 1 on */
+  /* the CFL minimum comes from k_plm_r (and dt from it, stored here for the
+   * phases before k_update stores it); PLM results are kept only from phase 1 on */
   CKK(dgk_rslope(&c->d, NULL, c->stream));
   CKK(dgk_plm_r(&c->d, NULL, sub, c->stream));
+  if (sub == 1) CKK(dgk_dt(&c->d, c->stream));
   CKK(dgk_source(&c->d, NULL, sub, c->stream));
   if (stop >= 2) {
     CKK(dgk_flux_phi(&c->d, NULL, sub, c->stream));

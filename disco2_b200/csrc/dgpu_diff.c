@@ -416,6 +416,7 @@ static int shadow_substep(struct dgpu_ctx *c, DevPtrs *h, cudaStream_t s, int su
   CKK(dgk_merge(h, sub, s));
   CKK(dgk_rslope(h, NULL, s));
   CKK(dgk_plm_r(h, NULL, sub, s));
+  if (sub == 1 && !h->form_dt) CKK(dgk_dt(h, s));
   CKK(dgk_source(h, NULL, sub, s));
   CKK(dgk_flux_phi(h, NULL, sub, s));
   CKK(dgk_flux_r(h, NULL, sub, s));
@@ -430,6 +431,7 @@ static int prep_substep(struct dgpu_ctx *c, DevPtrs *h, cudaStream_t s, int sub)
   CKK(dgk_merge(h, sub, s));
   CKK(dgk_rslope(h, NULL, s));
   CKK(dgk_plm_r(h, NULL, sub, s));
+  if (sub == 1) CKK(dgk_dt(h, s)); /* the reverse kernels read the stored dt */
   CKK(dgk_ann_consts(h, sub, s));
   return DGPU_OK;
 }
@@ -451,17 +453,20 @@ static int record_graph(struct dgpu_ctx *c, struct dgpu_diff *D, int which) {
     case G_STEP: /* one step and its dt into slot *idx, ++*idx */
       if (dctx_launch_step(c)) return -1;
       return dgk_step_end(&c->d, Dd->dtlog, Dd->d_idx, c->stream);
-    case G_OBJ_DT: /* the same with dt = dtin[*idx] */
-      if (dgk_cellprep(&c->d, NULL, 1, c->stream) || dgk_merge(&c->d, 1, c->stream) ||
-          dgk_rslope(&c->d, NULL, c->stream) || dgk_plm_r(&c->d, NULL, 1, c->stream) ||
-          dgk_set_dt(&c->d, Dd->dtin, Dd->d_idx, c->stream) || dgk_source(&c->d, NULL, 1, c->stream) ||
-          dgk_flux_phi(&c->d, NULL, 1, c->stream) || dgk_flux_r(&c->d, NULL, 1, c->stream) ||
-          dgk_update(&c->d, NULL, 1, 7, c->stream) || dctx_substep(c, NULL, 2, DCTX_FULL, NULL, NULL))
+    case G_OBJ_DT: { /* the same with dt = dtin[*idx] */
+      DevPtrs h = c->d;
+      h.form_dt = 0;
+      if (dgk_cellprep(&h, NULL, 1, c->stream) || dgk_merge(&h, 1, c->stream) ||
+          dgk_rslope(&h, NULL, c->stream) || dgk_plm_r(&h, NULL, 1, c->stream) ||
+          dgk_set_dt(&h, Dd->dtin, Dd->d_idx, c->stream) || dgk_source(&h, NULL, 1, c->stream) ||
+          dgk_flux_phi(&h, NULL, 1, c->stream) || dgk_flux_r(&h, NULL, 1, c->stream) ||
+          dgk_update(&h, NULL, 1, 7, c->stream) || dctx_substep(c, NULL, 2))
         return -1;
       if (dgk_objective(&c->d, NULL, Dd->o_part, Dd->o_val, NULL, Dd->d_idx, c->stream)) return -1;
       return dgk_step_end(&c->d, Dd->dtlog, Dd->d_idx, c->stream);
+    }
     case G_TAN: /* one tangent step */
-      if (dctx_substep(c, &Dd->t, 1, DCTX_FULL, NULL, NULL) || dctx_substep(c, &Dd->t, 2, DCTX_FULL, NULL, NULL))
+      if (dctx_substep(c, &Dd->t, 1) || dctx_substep(c, &Dd->t, 2))
         return -1;
       if (dgk_objective(&c->d, &Dd->t, Dd->o_part, Dd->o_val, Dd->o_dot, Dd->d_idx, c->stream)) return -1;
       return dgk_step_end(&c->d, Dd->dtlog, Dd->d_idx, c->stream);

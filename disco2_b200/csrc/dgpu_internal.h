@@ -164,6 +164,8 @@ typedef struct {
   double *fS;             /* [5][n_slots] r-face slopes (WR - WL)/(deltaR + deltaL) */
   double *fdp;            /* [2][n_slots] r-face offsets dpL, dpR (wrapped to [-pi, pi]) */
   double *ann_c;          /* [4][n_ann] per substep: kappa, cos(kappa dt), sin(kappa dt), 1-exp(-rate dt) */
+  int form_dt;            /* substep 1 forms dt from dtkey where it is read (step_dt); 0: dgk_dt or
+                             dgk_set_dt has stored it */
   int smem_face;          /* dynamic shared bytes of k_merge (0: merge reads global memory) */
   int merge_nt;           /* threads per k_merge / k_zmerge block (32..256) */
   int zghost;             /* cells of the ng lowest layers of the context's one 3-D disk, which
@@ -256,6 +258,9 @@ extern "C" {
  * launches the forward kernels, t != NULL their tangent instances. */
 int dgk_cellprep(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
 int dgk_merge(const DevPtrs *d, int substep, void *stream);
+/* stores each disk's dt from its CFL minimum (after plm_r of substep 1, for
+ * readers of InstState.dt) */
+int dgk_dt(const DevPtrs *d, void *stream);
 int dgk_source(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
 int dgk_rslope(const DevPtrs *d, const TanPtrs *t, void *stream);
 int dgk_plm_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);

@@ -11,8 +11,8 @@
 //                                 cell_plm_rz / riemann_setup_rz
 //   k_plm_r    per cell         : cell_plm_rz (face-weighted slope + limiter)
 //                                 and, in substep 1, the CFL minimum
-//                                 (cell_mindt); k_dt then forms dt
-//                                 (timestep_set_dt)
+//                                 (cell_mindt), from which dt is formed
+//                                 (timestep_set_dt: step_dt)
 //   k_source   per cell         : the increments of cell_add_src and
 //                                 cell_add_visc_src; per-annulus constants
 //   k_flux_phi per phi face     : riemann_setup_p + riemann_AddFlux
@@ -22,7 +22,7 @@
 //                                 accumulation order, cell_add_split_fictitious,
 //                                 cell_update_phi/_dphi, cell_calc_prim, the
 //                                 fixed radial boundary, cell_bc_damp and
-//                                 cell_calc_cons; its last block advances the
+//                                 cell_calc_cons; its first block advances the
 //                                 GravMass state
 // and, for disks with the outflow radial boundary, k_outflow per boundary cell
 // (cell_boundary_outflow_r).  k_merge runs beside k_cellprep on a second
@@ -65,6 +65,9 @@
 #ifndef DGPU_MINB_SWEEP
 #define DGPU_MINB_SWEEP 3
 #endif
+
+// Threads per block of k_plm_r, k_flux_phi, k_flux_r and k_update.
+#define TBLK 256
 
 namespace {
 
@@ -674,7 +677,7 @@ __device__ __forceinline__ unsigned long long cfl_key(const DevPtrs &d, const An
 }
 
 template <typename T, int MB = DGPU_MINB_PLM, bool PS = false>
-__global__ void __launch_bounds__(BLK, MB) k_plm_r(DevPtrs d, TanPtrs tp, int substep) {
+__global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_plm_r(DevPtrs d, TanPtrs tp, int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int N = d.n_cells;
   unsigned long long key = ~0ull;
@@ -718,16 +721,12 @@ __global__ void __launch_bounds__(BLK, MB) k_plm_r(DevPtrs d, TanPtrs tp, int su
   }
 }
 
-// dt of each disk once k_plm_r has formed the CFL minimum: the minimum,
-// clipped to Time_Max (timestep_set_dt, timestep_set.c:16-21).  A kernel of
-// its own, so that no block of k_plm_r has to wait for its stores to land
-// before a last block is elected.
+// Stores each disk's dt of substep 1, for readers of InstState.dt that run
+// before k_update does.
 __global__ void k_dt(DevPtrs d) {
   for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
     InstState &S = d.ist[k];
-    double dt = __longlong_as_double((long long)S.dtkey);
-    if (S.t + dt > d.par[k].t_max) dt = d.par[k].t_max - S.t;
-    S.dt = dt;
+    S.dt = cfl_dt(S, d.par[k]);
   }
 }
 
@@ -735,11 +734,10 @@ __global__ void k_dt(DevPtrs d) {
 // Face increments: one thread per phi face (at its left cell) and per r-face slot
 // ---------------------------------------------------------------------------
 // phi faces: thread per cell j, face (j, j+1) (riemann_setup_p, Riemann_setup.c:46-80)
-// S: the disk's state with this substep's GravMass positions; dt: the
-// substep's fac * dt.
+// ist: the disks' states with this substep's GravMass positions (NULL: d.ist).
 template <typename T, bool PS>
-__device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &tp, int g, const InstState &S,
-                                              double dt) {
+__device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &tp, int g, const InstState *ist,
+                                              int substep) {
   const int N = d.n_cells;
   // the cell's own planes (its right neighbour's share the lines) ahead of
   // the annulus lookups
@@ -773,7 +771,8 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
     qR[s] = ld(d.prim, 5 + s, N, cR) - 0.5 * ld(d.gradp, 5 + s, N, cR) * dpR;
   }
   riemann_flux(pL, pR, r, 1, w, P.gamma, P.riemann, F, np, qL, qR, Fq);
-  const double k = dt * dA;
+  const InstState &S = ist ? *ist : d.ist[A.inst];
+  const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
 #pragma unroll
   for (int q = 0; q < 5; ++q) stq<T>(d.fphi, tp.fphi, q, N, g, k * F[q]);
   for (int s = 0; s < np; ++s) d.fphi[(size_t)(8 + s) * N + g] = k * Fq[s];
@@ -804,17 +803,16 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
 }
 
 template <typename T, int MB = DGPU_MINB_FLUX, bool PS = false>
-__global__ void __launch_bounds__(BLK, MB) k_flux_phi(DevPtrs d, TanPtrs tp, int substep) {
+__global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_flux_phi(DevPtrs d, TanPtrs tp, int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.n_cells) return;
-  const InstState &S = d.ist[d.ann[d.cell_ann[g]].inst];
-  flux_phi_cell<T, PS>(d, tp, g, S, (substep == 1 ? 1.0 : 0.5) * S.dt);
+  flux_phi_cell<T, PS>(d, tp, g, nullptr, substep);
 }
 
 // r faces: thread per face slot (riemann_setup_rz, Riemann_setup.c:11-44)
 template <typename T, bool PS>
-__device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp, int slot, const InstState &S,
-                                            double dt) {
+__device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp, int slot, const InstState *ist,
+                                            int substep) {
   const int N = d.n_cells;
   const int cL = d.fL[slot];
   if (cL < 0) return;  // slot past the face list of its pair
@@ -846,7 +844,8 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
     qR[s] = ld(d.prim, 5 + s, N, cR) - ld(d.grad, 5 + s, N, cR) * deltaR - ld(d.gradp, 5 + s, N, cR) * dpR;
   }
   riemann_flux(pL, pR, r, 0, 0.0, P.gamma, P.riemann, F, np, qL, qR, Fq);
-  const double k = dt * dA;
+  const InstState &S = ist ? *ist : d.ist[A.inst];
+  const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
   const int NS = d.n_slots;
 #pragma unroll
   for (int q = 0; q < 5; ++q) stq<T>(d.frf, tp.frf, q, NS, slot, k * F[q]);
@@ -879,12 +878,10 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
 }
 
 template <typename T, int MB = DGPU_MINB_FLUXR, bool PS = false>
-__global__ void __launch_bounds__(BLK, MB) k_flux_r(DevPtrs d, TanPtrs tp, int substep) {
+__global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_flux_r(DevPtrs d, TanPtrs tp, int substep) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= d.n_slots) return;
-  if (d.fL[slot] < 0) return;  // slot past the face list of its pair
-  const InstState &S = d.ist[d.ann[d.slot_ann[slot]].inst];
-  flux_r_face<T, PS>(d, tp, slot, S, (substep == 1 ? 1.0 : 0.5) * S.dt);
+  flux_r_face<T, PS>(d, tp, slot, nullptr, substep);
 }
 
 // ---------------------------------------------------------------------------
@@ -989,7 +986,7 @@ __global__ void __launch_bounds__(BLK) k_flux_z(DevPtrs d, int substep) {
     pR[q] = ld(d.prim, q, N, cR) - ld(d.gradz, q, N, cR) * deltaR - ld(d.gradp, q, N, cR) * dpR;
   }
   riemann_flux(pL, pR, r, 2, 0.0, P.gamma, P.riemann, F);
-  const double k = fac * S.dt * dA;
+  const double k = fac * step_dt(d, S, P, substep) * dA;
 #pragma unroll
   for (int q = 0; q < 5; ++q) d.zfrf[(size_t)q * NS + slot] = k * F[q];
   if (P.has_visc) {
@@ -1173,13 +1170,15 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
   const int N = d.n_cells;
   const double fac = substep == 1 ? 1.0 : 0.5;
   if (t < d.n_ann) {
-    const InstState &S = d.ist[d.ann[t].inst];
-    ann_consts(d, t, S, fac * S.dt);
+    const int inst = d.ann[t].inst;
+    const InstState &S = d.ist[inst];
+    ann_consts(d, t, S, fac * step_dt(d, S, d.par[inst], substep));
   }
   double md0 = 0.0, md1 = 0.0;
   if (t < N && cells) {
-    const InstState &S = d.ist[d.ann[d.cell_ann[t]].inst];
-    source_cell_k<T, PS>(d, tp, t, S, fac * S.dt, md0, md1);
+    const int inst = d.ann[d.cell_ann[t]].inst;
+    const InstState &S = d.ist[inst];
+    source_cell_k<T, PS>(d, tp, t, S, fac * step_dt(d, S, d.par[inst], substep), md0, md1);
   }
   // deterministic per-block Mdot partial sums (reduced in block order by k_update)
   const unsigned full = 0xffffffffu;
@@ -1207,14 +1206,14 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
 // The update of cell g after its face and source increments are in place:
 // the conserved sum in the reference's order (update_sum),
 // cell_update_phi/_dphi, cell_calc_prim, the fixed radial boundary,
-// cell_bc_damp and cell_calc_cons.  dt: the substep's fac * dt.  XC: the
+// cell_bc_damp and cell_calc_cons.  ist: the disk's state (NULL: d.ist).  XC: the
 // increments were written by other blocks of the running kernel (plain loads,
 // not the read-only path).  rec (the adjoint's segment replay, else NULL): the
 // conserved sum before cons2prim and the new width of each cell go to slot
 // 2 * (*rec_idx) + substep - 1 of rec ([slot][6][n_cells]).
 template <typename T, bool PS, bool XC = false>
 __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp, int g, int substep, int stop,
-                                            double dt, double *rec, const int *rec_idx) {
+                                            const InstState *ist, double *rec, const int *rec_idx) {
   const int N = d.n_cells;
   {
     // the cell's own planes, before the annulus lookups they do not depend on
@@ -1233,6 +1232,7 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
     const int a = d.cell_ann[g];
     const Annulus &A = d.ann[a];
     const DiskParams &P = d.par[A.inst];
+    const double dt = (substep == 1 ? 1.0 : 0.5) * step_dt(d, ist ? *ist : d.ist[A.inst], P, substep);
     T c[5];
     double cp[DGPU_MAX_PASSIVE], pp[DGPU_MAX_PASSIVE];
     const int np = PS ? P.num_n : 0;
@@ -1343,45 +1343,38 @@ __device__ __forceinline__ void gm_tail(const DevPtrs &d, InstState &S, const Di
   }
 }
 
+// Every block updates cells; with tail > 0 block 0 moves the GravMass of every
+// disk instead, while the others work: no cell of this kernel reads what it
+// writes.  (A last block elected by a counter did it after all the others, a
+// chain of two pow at the end of every substep.)
 template <typename T, int MB = DGPU_MINB_UPDATE, bool PS = false>
-__global__ void __launch_bounds__(BLK, MB) k_update(DevPtrs d, TanPtrs tp, int substep, int stop,
+__global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, TanPtrs tp, int substep, int stop,
                                                                   int tail, double *rec, const int *rec_idx) {
-  __shared__ bool last;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells;
-  const double fac = substep == 1 ? 1.0 : 0.5;
-  if (g < N) {
-    const InstState &S = d.ist[d.ann[d.cell_ann[g]].inst];
-    update_cell<T, PS>(d, tp, g, substep, stop, fac * S.dt, rec, rec_idx);
-  }
-  if (tail == 0) return;
-  // the last block reads nothing the other blocks write (mdot_part comes from
-  // k_source), so no fence is needed before the count
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&d.counters[1], 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
-    InstState &S = d.ist[k];
-    const DiskParams &P = d.par[k];
-    // Mdot of this disk: block partials in block order
-    {
-      int c0 = P.cell_base, c1 = P.cell_base + P.n_cells;
-      int b0 = c0 / BLK, b1 = (c1 + BLK - 1) / BLK;
+  int b = blockIdx.x;
+  if (tail > 0 && b-- == 0) {
+    for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
+      InstState &S = d.ist[k];
+      const DiskParams &P = d.par[k];
+      if (substep == 1 && d.form_dt) S.dt = cfl_dt(S, P);
+      // Mdot of this disk: block partials in block order
+      const int c0 = P.cell_base, c1 = P.cell_base + P.n_cells;
+      const int b0 = c0 / BLK, b1 = (c1 + BLK - 1) / BLK;
       double s0 = 0.0, s1 = 0.0;
       if (P.rho_sink_on == 1) {
-        for (int b = b0; b < b1; ++b) {
-          s0 += d.mdot_part[2 * b];
-          s1 += d.mdot_part[2 * b + 1];
+        for (int m = b0; m < b1; ++m) {
+          s0 += d.mdot_part[2 * m];
+          s1 += d.mdot_part[2 * m + 1];
         }
       }
       S.mdot[0] = s0;
       S.mdot[1] = s1;
+      gm_tail(d, S, P, substep, tail);
     }
-    gm_tail(d, S, P, substep, tail);
+    return;
   }
-  if (threadIdx.x == 0) d.counters[1] = 0;
+  const int g = b * TBLK + threadIdx.x;
+  if (g >= d.n_cells) return;
+  update_cell<T, PS>(d, tp, g, substep, stop, nullptr, rec, rec_idx);
 }
 
 // ---------------------------------------------------------------------------
@@ -1456,7 +1449,7 @@ __global__ void __launch_bounds__(BLK, MB) k_prep(DevPtrs d, int substep) {
 
 // dt of a disk from k_prep's per-annulus CFL minima: the minimum (1e100 when
 // no cell has a candidate), clipped to Time_Max (timestep_set_dt,
-// src/TimeStep/timestep_set.c:16-21).  The same value as k_plm_r + k_dt form.
+// src/TimeStep/timestep_set.c:16-21).  The same value as cfl_dt forms from dtkey.
 __device__ __forceinline__ double sweep_dt(const DevPtrs &d, const DiskParams &P, double t) {
   unsigned long long key = (unsigned long long)__double_as_longlong(1.e100);
   for (int k = P.ann_base; k < P.ann_base + P.NR; ++k) {
@@ -1512,27 +1505,27 @@ SWEEP_FN void sweep_grad(const DevPtrs &d, int a) {
   const Annulus &A = d.ann[a];
   for (int j = threadIdx.x; j < A.np; j += BLK) plm_r_grad<double, false>(d, tp, A.cell_off + j);
 }
-SWEEP_FN void sweep_flux_r(const DevPtrs &d, int b, const InstState &S, double dt) {
+SWEEP_FN void sweep_flux_r(const DevPtrs &d, int b, const InstState &S, int substep) {
   const TanPtrs tp = {};
   const Annulus &Q = d.ann[b];
   const int nf = d.pair_nf[b];
-  for (int n = threadIdx.x; n < nf; n += BLK) flux_r_face<double, false>(d, tp, Q.face_base + n, S, dt);
+  for (int n = threadIdx.x; n < nf; n += BLK) flux_r_face<double, false>(d, tp, Q.face_base + n, &S, substep);
 }
-SWEEP_FN void sweep_cells(const DevPtrs &d, int a, const InstState &S, double dt) {
+SWEEP_FN void sweep_cells(const DevPtrs &d, int a, const InstState &S, int substep, double dt) {
   const TanPtrs tp = {};
   const Annulus &A = d.ann[a];
   double md0 = 0.0, md1 = 0.0;
   for (int j = threadIdx.x; j < A.np; j += BLK) {
     const int g = A.cell_off + j;
-    flux_phi_cell<double, false>(d, tp, g, S, dt);
+    flux_phi_cell<double, false>(d, tp, g, &S, substep);
     source_cell_k<double, false>(d, tp, g, S, dt, md0, md1);
   }
 }
-SWEEP_FN void sweep_update_cells(const DevPtrs &d, int b, int substep, double dt) {
+SWEEP_FN void sweep_update_cells(const DevPtrs &d, int b, int substep, const InstState &S) {
   const TanPtrs tp = {};
   const Annulus &B = d.ann[b];
   for (int j = threadIdx.x; j < B.np; j += BLK)
-    update_cell<double, false, true>(d, tp, B.cell_off + j, substep, 7, dt, nullptr, nullptr);
+    update_cell<double, false, true>(d, tp, B.cell_off + j, substep, 7, &S, nullptr, nullptr);
 }
 
 // The update of annulus b's cells (update_cell) once its increments are in
@@ -1540,7 +1533,7 @@ SWEEP_FN void sweep_update_cells(const DevPtrs &d, int b, int substep, double dt
 __device__ __forceinline__ void sweep_update(const DevPtrs &d, int b, int substep, const InstState &S, double dt) {
   if (threadIdx.x == 0) ann_consts(d, b, S, dt);
   __syncthreads();
-  sweep_update_cells(d, b, substep, dt);
+  sweep_update_cells(d, b, substep, S);
 }
 
 // k_sweep: the rest of the substep as one wavefront over the annuli.  Each
@@ -1596,9 +1589,9 @@ __global__ void __launch_bounds__(BLK, MB) k_sweep(const __grid_constant__ DevPt
   // 3. fluxes of pair (a-1, a); phi faces and sources of annulus a
   if (!first) {
     sweep_wait(d, a - 1, 2);
-    sweep_flux_r(d, a - 1, s_S, dt);
+    sweep_flux_r(d, a - 1, s_S, substep);
   }
-  sweep_cells(d, a, s_S, dt);
+  sweep_cells(d, a, s_S, substep, dt);
   sweep_publish(d, a, 3);
   // 4. update of annulus a-1, then of the disk's last annulus
   if (!first) {
@@ -1907,23 +1900,24 @@ int dgk_block_size(void) { return BLK; }
       kern<double, true><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, none_, __VA_ARGS__); \
     else kern<double><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, none_, __VA_ARGS__);    \
   } while (0)
-// The same for the kernels the autotuner sizes: the forward instance with
-// d->tune[which] resident blocks per SM (0: the built-in choice).
-#define DGK_LAUNCH_TUNED(kern, which, mbdef, grid, stream, ...)                           \
+// The same for the kernels the autotuner sizes, in blocks of blk threads: the
+// forward instance with d->tune[which] resident blocks of BLK threads per SM
+// (0: the built-in choice).
+#define DGK_LAUNCH_TUNED(kern, which, mbdef, grid, blk, stream, ...)                           \
   do {                                                                                   \
     static const TanPtrs none_ = {};                                                     \
     cudaStream_t s_ = (cudaStream_t)(stream);                                            \
     if (t) {                                                                             \
-      kern<Dual><<<(grid), BLK, 0, s_>>>(*d, *t, __VA_ARGS__);                            \
+      kern<Dual><<<(grid), blk, 0, s_>>>(*d, *t, __VA_ARGS__);                            \
     } else if (d->n_pass > 0) {                                                          \
-      kern<double, mbdef, true><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__);          \
+      kern<double, mbdef, true><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__);          \
     } else {                                                                             \
       switch (d->tune[which]) {                                                          \
-        case 2: kern<double, 2><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 3: kern<double, 3><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 4: kern<double, 4><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 5: kern<double, 5><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        default: kern<double><<<(grid), BLK, 0, s_>>>(*d, none_, __VA_ARGS__);           \
+        case 2: kern<double, 2><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+        case 3: kern<double, 3><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+        case 4: kern<double, 4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+        case 5: kern<double, 5><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+        default: kern<double><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__);           \
       }                                                                                  \
     }                                                                                    \
   } while (0)
@@ -1945,34 +1939,41 @@ int dgk_rslope(const DevPtrs *d, const TanPtrs *t, void *stream) {
   return (int)cudaGetLastError();
 }
 int dgk_plm_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) {
-  DGK_LAUNCH_TUNED(k_plm_r, DGPU_TUNE_PLM, DGPU_MINB_PLM, (d->n_cells + BLK - 1) / BLK, stream, substep);
-  if (substep == 1) k_dt<<<1, BLK, 0, (cudaStream_t)stream>>>(*d);
+  DGK_LAUNCH_TUNED(k_plm_r, DGPU_TUNE_PLM, DGPU_MINB_PLM, (d->n_cells + TBLK - 1) / TBLK, TBLK, stream, substep);
+  return (int)cudaGetLastError();
+}
+int dgk_dt(const DevPtrs *d, void *stream) {
+  k_dt<<<1, BLK, 0, (cudaStream_t)stream>>>(*d);
   return (int)cudaGetLastError();
 }
 int dgk_flux_phi(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) {
-  DGK_LAUNCH_TUNED(k_flux_phi, DGPU_TUNE_FLUXPHI, DGPU_MINB_FLUX, (d->n_cells + BLK - 1) / BLK, stream, substep);
+  DGK_LAUNCH_TUNED(k_flux_phi, DGPU_TUNE_FLUXPHI, DGPU_MINB_FLUX, (d->n_cells + TBLK - 1) / TBLK, TBLK, stream,
+                   substep);
   return (int)cudaGetLastError();
 }
 int dgk_flux_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) {
   if (d->n_slots <= 0) return 0;
-  DGK_LAUNCH_TUNED(k_flux_r, DGPU_TUNE_FLUXR, DGPU_MINB_FLUXR, (d->n_slots + BLK - 1) / BLK, stream, substep);
+  DGK_LAUNCH_TUNED(k_flux_r, DGPU_TUNE_FLUXR, DGPU_MINB_FLUXR, (d->n_slots + TBLK - 1) / TBLK, TBLK, stream,
+                   substep);
   return (int)cudaGetLastError();
 }
 int dgk_source(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) {
   int n = d->n_cells > d->n_ann ? d->n_cells : d->n_ann;
-  DGK_LAUNCH_TUNED(k_source, DGPU_TUNE_SOURCE, DGPU_MINB_SOURCE, (n + BLK - 1) / BLK, stream, substep, 1);
+  DGK_LAUNCH_TUNED(k_source, DGPU_TUNE_SOURCE, DGPU_MINB_SOURCE, (n + BLK - 1) / BLK, BLK, stream, substep, 1);
   return (int)cudaGetLastError();
 }
+// k_update's blocks: the cells', and the GravMass block with tail > 0
+static int update_grid(const DevPtrs *d, int tail) { return (d->n_cells + TBLK - 1) / TBLK + (tail > 0); }
 int dgk_update(const DevPtrs *d, const TanPtrs *t, int substep, int stop, void *stream) {
   int tail = stop >= 7 ? 2 : (stop >= 5 ? 1 : 0);
-  DGK_LAUNCH_TUNED(k_update, DGPU_TUNE_UPDATE, DGPU_MINB_UPDATE, dgk_update_blocks(d->n_cells), stream, substep, stop, tail,
+  DGK_LAUNCH_TUNED(k_update, DGPU_TUNE_UPDATE, DGPU_MINB_UPDATE, update_grid(d, tail), TBLK, stream, substep, stop, tail,
+                  
                    (double *)NULL, (const int *)NULL);
   return (int)cudaGetLastError();
 }
 int dgk_update_rec(const DevPtrs *d, int substep, double *rec, const int *rec_idx, void *stream) {
   static const TanPtrs none = {};
-  k_update<double><<<dgk_update_blocks(d->n_cells), BLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 7, 2, rec,
-                                                                                      rec_idx);
+  k_update<double><<<update_grid(d, 2), TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 7, 2, rec, rec_idx);
   return (int)cudaGetLastError();
 }
 int dgk_ann_consts(const DevPtrs *d, int substep, void *stream) {
@@ -1983,12 +1984,12 @@ int dgk_ann_consts(const DevPtrs *d, int substep, void *stream) {
 int dgk_update_stage(const DevPtrs *d, int substep, int stop, void *stream) {
   int tail = stop >= 5 ? 1 : 0;
   static const TanPtrs none = {};
+  const int nb = update_grid(d, tail);
   if (d->n_pass > 0)
-    k_update<double, DGPU_MINB_UPDATE, true><<<dgk_update_blocks(d->n_cells), BLK, 0, (cudaStream_t)stream>>>(
+    k_update<double, DGPU_MINB_UPDATE, true><<<nb, TBLK, 0, (cudaStream_t)stream>>>(
         *d, none, substep, stop, tail, nullptr, nullptr);
   else
-    k_update<double><<<dgk_update_blocks(d->n_cells), BLK, 0, (cudaStream_t)stream>>>(*d, none, substep, stop,
-                                                                                        tail, nullptr, nullptr);
+    k_update<double><<<nb, TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, stop, tail, nullptr, nullptr);
   return (int)cudaGetLastError();
 }
 int dgk_zmerge(const DevPtrs *d, int substep, void *stream) {

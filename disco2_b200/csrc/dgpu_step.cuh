@@ -35,6 +35,22 @@ __device__ __forceinline__ void grav_t(GravT<T> &G, const InstState &S, const Di
   }
 }
 
+// timestep_set_dt (timestep_set.c:16-21): the CFL minimum that k_plm_r left in
+// dtkey, clipped to Time_Max.
+__device__ __forceinline__ double cfl_dt(const InstState &S, const DiskParams &P) {
+  double dt = __longlong_as_double((long long)S.dtkey);
+  if (S.t + dt > P.t_max) dt = P.t_max - S.t;
+  return dt;
+}
+// dt of the disk's current step.  With form_dt every reader of substep 1 forms
+// it, so that no launch stands between k_plm_r and the fluxes for it (2.5 us of
+// a 120 us step); k_update's first block stores it.  A context of many waves
+// hides that launch and pays for the extra loads instead (12 disks, 3 M cells:
+// 4.48 against 4.45 ms a step), so there dgk_dt stores it first.
+__device__ __forceinline__ double step_dt(const DevPtrs &d, const InstState &S, const DiskParams &P, int substep) {
+  return substep == 1 && d.form_dt ? cfl_dt(S, P) : S.dt;
+}
+
 // Frame terms of annulus a in the substep: A_MILOS's depend on the binary's
 // separation, so they are formed once per annulus and substep (k_merge:
 // milos_frame) instead of by every cell and face -- five pow per term; the
