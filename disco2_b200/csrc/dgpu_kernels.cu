@@ -66,8 +66,12 @@
 #define DGPU_MINB_SWEEP 3
 #endif
 
-// Threads per block of k_plm_r, k_flux_phi, k_flux_r and k_update.
-#define TBLK 256
+// Threads per block of k_plm_r, k_flux_phi, k_flux_r and k_update: half of BLK
+// at the same registers per thread.  A block's registers are given back when
+// its slowest warp is done, so smaller blocks leave fewer of them idle (a step
+// of 16 disks, 4 M cells: 4.43 ms at 256, 4.37 at 128, 4.38-4.44 at 64; one
+// 258,078-cell disk 0.353, 0.351 and 0.353-0.367).
+#define TBLK 128
 
 namespace {
 
