@@ -2028,10 +2028,12 @@ int dgk_prep(const DevPtrs *d, int substep, void *stream) {
 }
 int dgk_sweep(const DevPtrs *d, int substep, void *stream) {
   cudaStream_t s_ = (cudaStream_t)stream;
+  DevPtrs h = *d;
+  h.form_dt = 0;  // its blocks hold the dt they form themselves (sweep_dt)
   switch (d->tune[DGPU_TUNE_SWEEP]) {
-    case 2: k_sweep<2><<<d->n_ann, BLK, 0, s_>>>(*d, substep); break;
-    case 4: k_sweep<4><<<d->n_ann, BLK, 0, s_>>>(*d, substep); break;
-    default: k_sweep<DGPU_MINB_SWEEP><<<d->n_ann, BLK, 0, s_>>>(*d, substep);
+    case 2: k_sweep<2><<<d->n_ann, BLK, 0, s_>>>(h, substep); break;
+    case 4: k_sweep<4><<<d->n_ann, BLK, 0, s_>>>(h, substep); break;
+    default: k_sweep<DGPU_MINB_SWEEP><<<d->n_ann, BLK, 0, s_>>>(h, substep);
   }
   return (int)cudaGetLastError();
 }
