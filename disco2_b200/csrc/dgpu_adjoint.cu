@@ -104,7 +104,6 @@ __device__ __forceinline__ void grav_adj_part(const GravAdj &ag, const double *c
 // accretion contribution -rho v_r r dphi dz (innermost non-ghost annulus).
 template <typename T>
 __device__ __forceinline__ void objective_cell(const DevPtrs &d, const TanPtrs &tp, int g, T &tq, T &md) {
-  const int N = d.n_cells;
   const Annulus A = d.ann[d.cell_ann[g]];
   const DiskParams &P = d.par[A.inst];
   const InstState &S = d.ist[A.inst];
@@ -114,7 +113,7 @@ __device__ __forceinline__ void objective_cell(const DevPtrs &d, const TanPtrs &
   md = 0.0;
   if (A.kind & DGPU_AK_CFL) {
     const double phi = d.tiph0[g] - .5 * dphi;
-    const T rho = ldq<T>(d.prim, tp.prim, D_RHO, N, g);
+    const T rho = ldq<T>(d.prim, tp.prim, D_RHO, P5, g);
     const double dV = dphi * .5 * A.dv_diff * P.dz;
     const double cosp = cos(phi), sinp = sin(phi);
     T Fp = 0.0;
@@ -138,8 +137,8 @@ __device__ __forceinline__ void objective_cell(const DevPtrs &d, const TanPtrs &
     tq = -(r * rho * dV * Fp);
   }
   if (A.kind & DGPU_AK_MDOT) {
-    const T rho = ldq<T>(d.prim, tp.prim, D_RHO, N, g);
-    const T vr = ldq<T>(d.prim, tp.prim, D_URR, N, g);
+    const T rho = ldq<T>(d.prim, tp.prim, D_RHO, P5, g);
+    const T vr = ldq<T>(d.prim, tp.prim, D_URR, P5, g);
     md = -(rho * vr * r * dphi * d.par[A.inst].dz);
   }
 }
@@ -202,25 +201,21 @@ __global__ void k_add_int(int *p, int dv) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *p += dv;
 }
 
-// Stored states: 19 doubles per cell (prim, cons, rkcons, tiph0, tiph1,
-// rktiph, dphi) and the disk states.  save: context -> store; else back.
-// A stored state: prim, cons, rkcons (5 planes each), tiph0, tiph1, rktiph,
-// dphi, then the passive-scalar planes of prim, cons and rkcons (n_pass each).
+// A stored state: prim, cons and rkcons (qs planes over n_pad cells each), then
+// tiph0, tiph1, rktiph and dphi (n_cells each), and the disk states.  save:
+// context -> store; else back.
 __device__ __forceinline__ void snap_copy_dev(const DevPtrs &d, double *sb, InstState *si, int save) {
-  const size_t N = (size_t)d.n_cells, NP = (size_t)d.n_pass * N;
-  const size_t n = 19 * N + 3 * NP;
+  const size_t N = (size_t)d.n_cells, M = (size_t)d.qs * d.n_pad;
+  const size_t n = 3 * M + 4 * N;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double *c;
-    if (i < 5 * N) c = d.prim + i;
-    else if (i < 10 * N) c = d.cons + (i - 5 * N);
-    else if (i < 15 * N) c = d.rkcons + (i - 10 * N);
-    else if (i < 16 * N) c = d.tiph0 + (i - 15 * N);
-    else if (i < 17 * N) c = d.tiph1 + (i - 16 * N);
-    else if (i < 18 * N) c = d.rktiph + (i - 17 * N);
-    else if (i < 19 * N) c = d.dphi + (i - 18 * N);
-    else if (i < 19 * N + NP) c = d.prim + 5 * N + (i - 19 * N);
-    else if (i < 19 * N + 2 * NP) c = d.cons + 5 * N + (i - 19 * N - NP);
-    else c = d.rkcons + 5 * N + (i - 19 * N - 2 * NP);
+    if (i < M) c = d.prim + i;
+    else if (i < 2 * M) c = d.cons + (i - M);
+    else if (i < 3 * M) c = d.rkcons + (i - 2 * M);
+    else if (i < 3 * M + N) c = d.tiph0 + (i - 3 * M);
+    else if (i < 3 * M + 2 * N) c = d.tiph1 + (i - 3 * M - N);
+    else if (i < 3 * M + 3 * N) c = d.rktiph + (i - 3 * M - 2 * N);
+    else c = d.dphi + (i - 3 * M - 3 * N);
     if (save) sb[i] = *c;
     else *c = sb[i];
   }
@@ -255,7 +250,8 @@ __global__ void __launch_bounds__(BLK) a_objective(DevPtrs d, AdjPtrs J, double 
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int N = d.n_cells;
   const double *sb = bufs[*idx + off];
-  const double *prim = sb, *tiph0 = sb + 15 * (size_t)N, *dphiv = sb + 18 * (size_t)N;
+  // (snap_copy_dev's layout; a differentiated context has 5 state planes)
+  const double *prim = sb, *tiph0 = sb + 15 * (size_t)d.n_pad, *dphiv = tiph0 + 3 * (size_t)N;
   const int n = *base + *idx;
   const double wT = wts[2 * n], wM = wts[2 * n + 1];
   double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -267,7 +263,7 @@ __global__ void __launch_bounds__(BLK) a_objective(DevPtrs d, AdjPtrs J, double 
     const double r = .5 * (A.rp + A.rm);
     if ((A.kind & DGPU_AK_CFL) && wT != 0.0) {
       const double phi = tiph0[g] - .5 * dphi;
-      const double rho = ld(prim, D_RHO, N, g);
+      const double rho = ld(prim, D_RHO, P5, g);
       const double dV = dphi * .5 * A.dv_diff * P.dz;
       const double cosp = cos(phi), sinp = sin(phi);
       double Fp = 0.0, f1[2], sinap[2], dx[2], dy[2], sr[2], cosa[2], sina[2], cg[2], sg[2];
@@ -284,7 +280,7 @@ __global__ void __launch_bounds__(BLK) a_objective(DevPtrs d, AdjPtrs J, double 
         Fp += sinap[p] * f1[p];
       }
       // tq = -(r rho dV Fp)
-      J.lW[(size_t)D_RHO * N + g] += -wT * r * dV * Fp;
+      J.lW[ix(D_RHO, P5, g)] += -wT * r * dV * Fp;
       const double aFp = -wT * r * rho * dV;
       for (int p = 0; p < 2; ++p) {
         const double asinap = aFp * f1[p], af1 = aFp * sinap[p];
@@ -302,10 +298,10 @@ __global__ void __launch_bounds__(BLK) a_objective(DevPtrs d, AdjPtrs J, double 
       }
     }
     if ((A.kind & DGPU_AK_MDOT) && wM != 0.0) {
-      const double rho = ld(prim, D_RHO, N, g), vr = ld(prim, D_URR, N, g);
+      const double rho = ld(prim, D_RHO, P5, g), vr = ld(prim, D_URR, P5, g);
       const double k = r * dphi * P.dz;
-      J.lW[(size_t)D_RHO * N + g] += -wM * vr * k;
-      J.lW[(size_t)D_URR * N + g] += -wM * rho * k;
+      J.lW[ix(D_RHO, P5, g)] += -wM * vr * k;
+      J.lW[ix(D_URR, P5, g)] += -wM * rho * k;
     }
   }
   block_partial<5>(v, J.part + DGPU_AP_N * (size_t)(row0 + blockIdx.x));
@@ -345,11 +341,10 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
     {
       // the conserved sum before cons2prim and the new width, recorded by the
       // segment replay's k_update
-      const double *rs = rec + (size_t)(2 * (*idx) + substep - 1) * 6 * N;
-      double c[5];
-#pragma unroll
-      for (int q = 0; q < 5; ++q) c[q] = rs[(size_t)q * N + g];
-      const double dphi_n = rs[(size_t)5 * N + g];
+      const double *rs = rec + (size_t)(2 * (*idx) + substep - 1) * 6 * d.n_pad;
+      double c[6];
+      ldk<6, true>(rs, 0, P6, g, c);
+      const double dphi_n = c[5];
       const double dV = A.dv_half * dphi_n * P.dz;
       double pr[5];
       cons2prim(c, dV, r, P, pr);
@@ -357,8 +352,8 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
       double apr[5], alc[5];
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        apr[q] = J.lW[(size_t)q * N + g];
-        alc[q] = J.lC[(size_t)q * N + g];
+        apr[q] = J.lW[ix(q, P5, g)];
+        alc[q] = J.lC[ix(q, P5, g)];
       }
       prim2cons_rev(pr, r, dV, P.gamma, alc, apr);
       if (P.has_damp && (A.kind & DGPU_AK_DAMP) && (A.kind & DGPU_AK_IC)) {
@@ -383,11 +378,11 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
     }
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      J.lU[(size_t)q * N + g] = ac[q];
+      J.lU[ix(q, P5, g)] = ac[q];
       double lc = (1.0 - RK) * ac[q];
-      if (substep == 1) lc += J.lCrk[(size_t)q * N + g];
-      else J.lCrk[(size_t)q * N + g] = RK * ac[q];
-      J.lC[(size_t)q * N + g] = lc;
+      if (substep == 1) lc += J.lCrk[ix(q, P5, g)];
+      else J.lCrk[ix(q, P5, g)] = RK * ac[q];
+      J.lC[ix(q, P5, g)] = lc;
     }
     // k_source reversed
     const double dphi = d.dphi[g];
@@ -419,11 +414,11 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
     grav_t(G, S, P, none, A.inst);
     double pm[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) pm[q] = ld(d.prim, q, N, g);
+    for (int q = 0; q < 5; ++q) pm[q] = ld(d.prim, q, P5, g);
     double gu = 0.0, gpu = 0.0;
     if (P.has_visc) {
-      gu = ld(d.grad, D_UPP, N, g);
-      gpu = ld(d.gradp, D_URR, N, g);
+      gu = ld(d.grad, D_UPP, P5, g);
+      gpu = ld(d.gradp, D_URR, P5, g);
     }
     double as[6];
     as[0] = as[1] = ac[D_SRR];
@@ -437,22 +432,24 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
     source_cell_rev(sg, P, pm, gu, gpu, G, as, apm, agu, agpu, ag);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      J.lWt[(size_t)q * N + g] = apm[q];
-      J.lG[(size_t)q * N + g] = q == D_UPP ? agu : 0.0;
-      J.lGp[(size_t)q * N + g] = q == D_URR ? agpu : 0.0;
+      J.lWt[ix(q, P5, g)] = apm[q];
+      J.lG[ix(q, P5, g)] = q == D_UPP ? agu : 0.0;
+      J.lGp[ix(q, P5, g)] = q == D_URR ? agpu : 0.0;
     }
     grav_adj_part(ag, S.gc, S.gs, v);
   }
   block_partial<5>(v, J.part + DGPU_AP_N * (size_t)(row0 + blockIdx.x));
 }
 
-__device__ __forceinline__ void store15(double *arr, int n, int i, const double *w, const double *gp, const double *gr) {
+__device__ __forceinline__ void store15(double *arr, int i, const double *w, const double *gp, const double *gr) {
+  double u[15];
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    arr[(size_t)q * n + i] = w[q];
-    arr[(size_t)(5 + q) * n + i] = gp[q];
-    arr[(size_t)(10 + q) * n + i] = gr[q];
+    u[q] = w[q];
+    u[5 + q] = gp[q];
+    u[10 + q] = gr[q];
   }
+  stk<15>(arr, 0, P15, i, u);
 }
 
 __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_phi(DevPtrs d, AdjPtrs J, int substep, int row0) {
@@ -473,13 +470,13 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_phi(DevPtrs d, AdjP
     double pL[5], pR[5], aF[5], aFv[3];
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      pL[q] = ld(d.prim, q, N, cL) + 0.5 * ld(d.gradp, q, N, cL) * dpL;
-      pR[q] = ld(d.prim, q, N, cR) - 0.5 * ld(d.gradp, q, N, cR) * dpR;
-      aF[q] = k * (ld(J.lU, q, N, cR) - ld(J.lU, q, N, cL));
+      pL[q] = ld(d.prim, q, P5, cL) + 0.5 * ld(d.gradp, q, P5, cL) * dpL;
+      pR[q] = ld(d.prim, q, P5, cR) - 0.5 * ld(d.gradp, q, P5, cR) * dpR;
+      aF[q] = k * (ld(J.lU, q, P5, cR) - ld(J.lU, q, P5, cL));
     }
-    aFv[0] = k * ((ld(J.lU, D_SRR, N, cR) - ld(J.lU, D_SRR, N, cL)) / r);
-    aFv[1] = k * (ld(J.lU, D_LLL, N, cR) - ld(J.lU, D_LLL, N, cL));
-    aFv[2] = k * (ld(J.lU, D_TAU, N, cR) - ld(J.lU, D_TAU, N, cL));
+    aFv[0] = k * ((ld(J.lU, D_SRR, P5, cR) - ld(J.lU, D_SRR, P5, cL)) / r);
+    aFv[1] = k * (ld(J.lU, D_LLL, P5, cR) - ld(J.lU, D_LLL, P5, cL));
+    aFv[2] = k * (ld(J.lU, D_TAU, P5, cR) - ld(J.lU, D_TAU, P5, cL));
     double apL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, apR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     riemann_flux_rev(pL, pR, r, 1, d.w_ann[a], P.gamma, P.riemann, aF, apL, apR);
     double wL[5], wR[5], gpL[5], gpR[5], grL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, grR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -494,11 +491,11 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_phi(DevPtrs d, AdjP
       ViscIn<double> vi;
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        vi.cL[q] = ld(d.prim, q, N, cL);
-        vi.cR[q] = ld(d.prim, q, N, cR);
+        vi.cL[q] = ld(d.prim, q, P5, cL);
+        vi.cR[q] = ld(d.prim, q, P5, cR);
         vi.gpL[q] = vi.gpR[q] = 0.0;
-        vi.grL[q] = ld(d.grad, q, N, cL);
-        vi.grR[q] = ld(d.grad, q, N, cR);
+        vi.grL[q] = ld(d.grad, q, P5, cL);
+        vi.grR[q] = ld(d.grad, q, P5, cR);
       }
       vi.tL = d.tiphw[cL];
       vi.tR = d.tiphw[cR];
@@ -525,15 +522,15 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_phi(DevPtrs d, AdjP
       }
       grav_adj_part(ag, S.gc, S.gs, v);
     }
-    store15(J.aphiL, N, g, wL, gpL, grL);
-    store15(J.aphiR, N, g, wR, gpR, grR);
+    store15(J.aphiL, g, wL, gpL, grL);
+    store15(J.aphiR, g, wR, gpR, grR);
   }
   block_partial<5>(v, J.part + DGPU_AP_N * (size_t)(row0 + blockIdx.x));
 }
 
 __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_r(DevPtrs d, AdjPtrs J, int substep, int row0) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells, NS = d.n_slots;
+  const int NS = d.n_slots;
   double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int cL = slot < NS ? d.fL[slot] : -1;
   if (cL >= 0) {
@@ -544,20 +541,22 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_r(DevPtrs d, AdjPtr
     const InstState &S = d.ist[A.inst];
     const double fac = substep == 1 ? 1.0 : 0.5;
     const double deltaL = A.f_dl, deltaR = A.f_dr;
-    const double dpL = d.fdp[slot], dpR = d.fdp[(size_t)NS + slot];
+    double dp[2];
+    ldk<2, true>(d.fdp, 0, P2, slot, dp);
+    const double dpL = dp[0], dpR = dp[1];
     const double r = A.f_r;
     const double k = fac * S.dt * (r * d.fdphi[slot] * A.f_dperp);
     const double rL = r - deltaL, rR = r + deltaR;
     double pL[5], pR[5], aF[5], aFv[3];
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      pL[q] = ld(d.prim, q, N, cL) + ld(d.grad, q, N, cL) * deltaL + ld(d.gradp, q, N, cL) * dpL;
-      pR[q] = ld(d.prim, q, N, cR) - ld(d.grad, q, N, cR) * deltaR - ld(d.gradp, q, N, cR) * dpR;
-      aF[q] = k * (ld(J.lU, q, N, cR) - ld(J.lU, q, N, cL));
+      pL[q] = ld(d.prim, q, P5, cL) + ld(d.grad, q, P5, cL) * deltaL + ld(d.gradp, q, P5, cL) * dpL;
+      pR[q] = ld(d.prim, q, P5, cR) - ld(d.grad, q, P5, cR) * deltaR - ld(d.gradp, q, P5, cR) * dpR;
+      aF[q] = k * (ld(J.lU, q, P5, cR) - ld(J.lU, q, P5, cL));
     }
-    aFv[0] = k * (ld(J.lU, D_SRR, N, cR) / rR - ld(J.lU, D_SRR, N, cL) / rL);
-    aFv[1] = k * (ld(J.lU, D_LLL, N, cR) - ld(J.lU, D_LLL, N, cL));
-    aFv[2] = k * (ld(J.lU, D_TAU, N, cR) - ld(J.lU, D_TAU, N, cL));
+    aFv[0] = k * (ld(J.lU, D_SRR, P5, cR) / rR - ld(J.lU, D_SRR, P5, cL) / rL);
+    aFv[1] = k * (ld(J.lU, D_LLL, P5, cR) - ld(J.lU, D_LLL, P5, cL));
+    aFv[2] = k * (ld(J.lU, D_TAU, P5, cR) - ld(J.lU, D_TAU, P5, cL));
     double apL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, apR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     riemann_flux_rev(pL, pR, r, 0, 0.0, P.gamma, P.riemann, aF, apL, apR);
     double wL[5], wR[5], gpL[5], gpR[5], grL[5], grR[5];
@@ -574,10 +573,10 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_r(DevPtrs d, AdjPtr
       ViscIn<double> vi;
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        vi.cL[q] = ld(d.prim, q, N, cL);
-        vi.cR[q] = ld(d.prim, q, N, cR);
-        vi.gpL[q] = ld(d.gradp, q, N, cL);
-        vi.gpR[q] = ld(d.gradp, q, N, cR);
+        vi.cL[q] = ld(d.prim, q, P5, cL);
+        vi.cR[q] = ld(d.prim, q, P5, cR);
+        vi.gpL[q] = ld(d.gradp, q, P5, cL);
+        vi.gpR[q] = ld(d.gradp, q, P5, cR);
         vi.grL[q] = vi.grR[q] = 0.0;
       }
       vi.tL = d.tiphw[cL];
@@ -606,8 +605,8 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_r(DevPtrs d, AdjPtr
       }
       grav_adj_part(ag, S.gc, S.gs, v);
     }
-    store15(J.arL, NS, slot, wL, gpL, grL);
-    store15(J.arR, NS, slot, wR, gpR, grR);
+    store15(J.arL, slot, wL, gpL, grL);
+    store15(J.arR, slot, wR, gpR, grR);
   }
   block_partial<5>(v, J.part + DGPU_AP_N * (size_t)(row0 + blockIdx.x));
 }
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_flux_r(DevPtrs d, AdjPtr
 // (src/Cell/cell_plm.c:81-113) onto the face slopes, replaying its branch.
 __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells, NS = d.n_slots;
+  const int N = d.n_cells;
   if (g >= N) return;
   const int a = d.cell_ann[g];
   const Annulus A = d.ann[a];
@@ -627,21 +626,21 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   double acc[15];
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    acc[q] = ld(J.lWt, q, N, g);
-    acc[5 + q] = ld(J.lGp, q, N, g);
-    acc[10 + q] = ld(J.lG, q, N, g);
+    acc[q] = ld(J.lWt, q, P5, g);
+    acc[5 + q] = ld(J.lGp, q, P5, g);
+    acc[10 + q] = ld(J.lG, q, P5, g);
   }
 #pragma unroll
-  for (int q = 0; q < 15; ++q) acc[q] += ld(J.aphiL, q, N, g) + ld(J.aphiR, q, N, gl);
+  for (int q = 0; q < 15; ++q) acc[q] += ld(J.aphiL, q, P15, g) + ld(J.aphiR, q, P15, gl);
   for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int asR) {
     const double *src = asR ? J.arR : J.arL;
 #pragma unroll
-    for (int q = 0; q < 15; ++q) acc[q] += ld(src, q, NS, slot);
+    for (int q = 0; q < 15; ++q) acc[q] += ld(src, q, P15, slot);
   });
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    J.lWt[(size_t)q * N + g] = acc[q];
-    J.lGp[(size_t)q * N + g] = acc[5 + q];
+    J.lWt[ix(q, P5, g)] = acc[q];
+    J.lGp[ix(q, P5, g)] = acc[5 + q];
   }
   // limiter replay: gq = sum S dA / dAtot, then per face (forward order):
   // zero if the face slope opposes, clip to plm * S if smaller
@@ -650,7 +649,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int) {
     double dA = F.r * F.dphi * F.dperp;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) gq[q] += ld(d.fS, q, NS, slot) * dA;
+    for (int q = 0; q < 5; ++q) gq[q] += ld(d.fS, q, P5, slot) * dA;
   });
   double dAtot;
   {
@@ -664,7 +663,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int) {
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      double Sq = ld(d.fS, q, NS, slot);
+      double Sq = ld(d.fS, q, P5, slot);
       if (Sq * gq[q] < 0.0) {
         gq[q] = 0.0;
         sel[q] = -2;
@@ -683,7 +682,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
       double w = 0.0;
       if (sel[q] == -1) w = lg * dA / dAtot;
       else if (sel[q] == slot) w = P.plm * lg;
-      dst[(size_t)q * NS + slot] = w;
+      dst[ix(q, P5, slot)] = w;
     }
   });
 }
@@ -692,7 +691,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
 // and phi slopes of each cell (its faces in the forward order).
 __global__ void __launch_bounds__(BLK) a_rslope(DevPtrs d, AdjPtrs J) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells, NS = d.n_slots;
+  const int N = d.n_cells;
   if (g >= N) return;
   const int a = d.cell_ann[g];
   const Annulus A = d.ann[a];
@@ -700,15 +699,15 @@ __global__ void __launch_bounds__(BLK) a_rslope(DevPtrs d, AdjPtrs J) {
   double lw[5], lgp[5];
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    lw[q] = ld(J.lWt, q, N, g);
-    lgp[q] = ld(J.lGp, q, N, g);
+    lw[q] = ld(J.lWt, q, P5, g);
+    lgp[q] = ld(J.lGp, q, P5, g);
   }
   for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int asR) {
     const double den = F.dr + F.dl;
-    const double dp = asR ? d.fdp[(size_t)NS + slot] : d.fdp[slot];
+    const double dp = ld(d.fdp, asR, P2, slot);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      const double ls = (ld(J.fsL, q, NS, slot) + ld(J.fsR, q, NS, slot)) / den;
+      const double ls = (ld(J.fsL, q, P5, slot) + ld(J.fsR, q, P5, slot)) / den;
       if (asR) lw[q] += ls;
       else lw[q] -= ls;
       lgp[q] -= dp * ls;
@@ -716,8 +715,8 @@ __global__ void __launch_bounds__(BLK) a_rslope(DevPtrs d, AdjPtrs J) {
   });
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    J.lWt[(size_t)q * N + g] = lw[q];
-    J.lGp[(size_t)q * N + g] = lgp[q];
+    J.lWt[ix(q, P5, g)] = lw[q];
+    J.lGp[ix(q, P5, g)] = lgp[q];
   }
 }
 
@@ -738,7 +737,7 @@ __global__ void __launch_bounds__(BLK) a_cellprep(DevPtrs d, AdjPtrs J) {
   (void)j;
   double lw[5];
 #pragma unroll
-  for (int q = 0; q < 5; ++q) lw[q] = ld(J.lWt, q, N, g);
+  for (int q = 0; q < 5; ++q) lw[q] = ld(J.lWt, q, P5, g);
   for (int m = 0; m < nk; ++m) {
     const int kk = ks[m], kl = left(kk), kr = right(kk);
     const double dc = d.dphi[kk];
@@ -747,14 +746,14 @@ __global__ void __launch_bounds__(BLK) a_cellprep(DevPtrs d, AdjPtrs J) {
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
       double cl, cc, cr;
-      plm_p_slope_coef(ld(d.prim, q, N, kl), ld(d.prim, q, N, kk), ld(d.prim, q, N, kr), dpL, dpR, P.plm, &cl, &cc,
+      plm_p_slope_coef(ld(d.prim, q, P5, kl), ld(d.prim, q, P5, kk), ld(d.prim, q, P5, kr), dpL, dpR, P.plm, &cl, &cc,
                        &cr);
       const double w = (kk == g ? cc : 0.0) + (kl == g ? cl : 0.0) + (kr == g ? cr : 0.0);
-      lw[q] += w * ld(J.lGp, q, N, kk);
+      lw[q] += w * ld(J.lGp, q, P5, kk);
     }
   }
 #pragma unroll
-  for (int q = 0; q < 5; ++q) J.lW[(size_t)q * N + g] = lw[q];
+  for (int q = 0; q < 5; ++q) J.lW[ix(q, P5, g)] = lw[q];
 }
 
 // cell_calc_cons reversed: lW += (d cons / d prim)^T lC on the current state.
@@ -769,13 +768,13 @@ __global__ void __launch_bounds__(BLK) a_calc_cons(DevPtrs d, AdjPtrs J) {
   double p[5], ac[5], ap[5];
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    p[q] = ld(d.prim, q, N, g);
-    ac[q] = ld(J.lC, q, N, g);
+    p[q] = ld(d.prim, q, P5, g);
+    ac[q] = ld(J.lC, q, P5, g);
     ap[q] = 0.0;
   }
   prim2cons_rev(p, r, dV, P.gamma, ac, ap);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) J.lW[(size_t)q * N + g] += ap[q];
+  for (int q = 0; q < 5; ++q) J.lW[ix(q, P5, g)] += ap[q];
 }
 
 }  // namespace
@@ -809,7 +808,7 @@ int dgk_add_int(int *p, int dv, void *stream) {
 }
 
 static int snap_grid(const DevPtrs *d) {
-  long long n = (19LL + 3LL * d->n_pass) * d->n_cells;
+  long long n = 3LL * d->qs * d->n_pad + 4LL * d->n_cells;
   long long b = (n + BLK - 1) / BLK;
   return (int)(b < 148 * 8 ? b : 148 * 8);
 }

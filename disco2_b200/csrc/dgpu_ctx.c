@@ -381,8 +381,12 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   }
   c->n_pass = n_pass;
   {
-    size_t N = (size_t)c->n_cells, S = (size_t)c->n_slots, A = (size_t)c->n_ann;
+    /* N, S: several-plane arrays of whole tiles; the single-plane ones take the same */
+    size_t N = DGPU_PAD(c->n_cells), S = DGPU_PAD(c->n_slots), A = (size_t)c->n_ann;
     const size_t NQ = 5 + (size_t)n_pass, NF = 8 + (size_t)n_pass;
+    c->d.n_pad = (int)N;
+    c->d.qs = (int)NQ;
+    c->d.qf = (int)NF;
     c->d_par = (DiskParams *)dmalloc(sizeof(DiskParams) * (size_t)n, &ok);
     c->d_ist = (InstState *)dmalloc(sizeof(InstState) * (size_t)n, &ok);
     c->d_ann = (Annulus *)dmalloc(sizeof(Annulus) * A, &ok);
@@ -422,7 +426,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
     c->d.cfl_ann = (unsigned long long *)dmalloc(sizeof(unsigned long long) * A, &ok);
     c->d.sweep_flag = (int *)dmalloc(sizeof(int) * A, &ok);
     if (has_z) {
-      const size_t ZS = (size_t)(zslots > 0 ? zslots : 1);
+      const size_t ZS = DGPU_PAD(zslots > 0 ? zslots : 1);
       c->d_zslot_ann = (int *)dmalloc(sizeof(int) * ZS, &ok);
       c->d.zfL = (int *)dmalloc(sizeof(int) * ZS, &ok);
       c->d.zfR = (int *)dmalloc(sizeof(int) * ZS, &ok);
@@ -588,7 +592,7 @@ static int upload_disk(struct dgpu_ctx *c, int inst, const double *prim, const d
   if (prim) {
     const int nq = 5 + p->num_n;
     CK(cudaMemcpyAsync(c->d_stage, prim, sizeof(double) * nq * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    CKK(dgk_aos_to_soa(c->d.prim, nq, c->n_cells, base, c->d_stage, n, c->stream));
+    CKK(dgk_aos_to_soa(c->d.prim, nq, c->d.qs, base, c->d_stage, n, c->stream));
   }
   if (tiph) CK(cudaMemcpyAsync(c->d.tiph0 + base, tiph, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
   if (dphi) CK(cudaMemcpyAsync(c->d.dphi + base, dphi, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
@@ -612,13 +616,13 @@ int dgpu_get_state(dgpu_ctx *c, int inst, double *prim, double *cons, double *ti
   n = p->n_cells;
   base = p->cell_base;
   if (prim) {
-    CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->n_cells, base, c->d.prim, n, c->stream));
+    CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->d.qs, base, c->d.prim, n, c->stream));
     CK(cudaMemcpyAsync(prim, c->d_stage, sizeof(double) * (5 + p->num_n) * (size_t)n, cudaMemcpyDeviceToHost,
                        c->stream));
     if (cons) CK(cudaStreamSynchronize(c->stream));
   }
   if (cons) {
-    CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->n_cells, base, c->d.cons, n, c->stream));
+    CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->d.qs, base, c->d.cons, n, c->stream));
     CK(cudaMemcpyAsync(cons, c->d_stage, sizeof(double) * (5 + p->num_n) * (size_t)n, cudaMemcpyDeviceToHost,
                        c->stream));
   }
@@ -641,7 +645,7 @@ int dgpu_get_stage_data(dgpu_ctx *c, int inst, double *grad, double *gradp, doub
     int k;
     for (k = 0; k < 3; ++k) {
       if (!dsts[k]) continue;
-      CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->n_cells, base, srcs[k], n, c->stream));
+      CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->d.qs, base, srcs[k], n, c->stream));
       CK(cudaMemcpyAsync(dsts[k], c->d_stage, sizeof(double) * (5 + p->num_n) * (size_t)n, cudaMemcpyDeviceToHost,
                          c->stream));
       CK(cudaStreamSynchronize(c->stream));
@@ -1000,7 +1004,7 @@ int dgpu_autotune(dgpu_ctx *c, int steps, int *choice) {
     for (k = 0; k < DGPU_TUNE_N; ++k) c->d.tune[k] = choice[k];
   } else {
     /* save the state, time each candidate from it, restore it */
-    if (cudaMalloc((void **)&buf, sizeof(double) * (19 + 3 * (size_t)c->n_pass) * (size_t)c->n_cells) != cudaSuccess ||
+    if (cudaMalloc((void **)&buf, sizeof(double) * (3 * (size_t)c->d.qs * (size_t)c->d.n_pad + 4 * (size_t)c->n_cells)) != cudaSuccess ||
         cudaMalloc((void **)&ist, sizeof(InstState) * (size_t)c->n_inst) != cudaSuccess) {
       cudaFree(buf);
       cudaGetLastError();

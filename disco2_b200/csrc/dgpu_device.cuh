@@ -21,6 +21,7 @@
 #include <climits>
 #include <math.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "dgpu_internal.h"
 
@@ -125,10 +126,24 @@ template <> struct Fld<Dual> {
   static HD Dual mk(double v, double d) { return Dual(v, d); }
 };
 
-HD double ld(const double *p, int q, int n, int g) { return p[(size_t)q * n + g]; }
+// Arrays of several variables ("planes") per cell or face, 32 cells at a time:
+// plane q of cell g is at ix(q, n, g), the 32 cells of a tile holding plane 0,
+// then plane 1, and so on, each 256 consecutive bytes.  The planes of a cell
+// are at constant distances from one address, which the load and store
+// instructions carry, so a plane costs no address arithmetic; with each plane
+// whole after the other every plane of every array did.
+// n: the array's planes (a type of its own, so that a cell count cannot stand
+// in for it).  Arrays are padded to whole tiles.
+struct Pl {
+  int n;
+};
+constexpr Pl P2 = {2}, P5 = {5}, P6 = {6}, P8 = {8}, P15 = {15};
+HD size_t ix(int q, Pl n, int g) { return (size_t)(g >> 5) * (size_t)(n.n * 32) + (size_t)(q * 32 + (g & 31)); }
+
+HD double ld(const double *p, int q, Pl n, int g) { return p[ix(q, n, g)]; }
 template <typename T>
-HD T ldq(const double *v, const double *d, int q, int n, int g) {
-  return Fld<T>::ld(v, d, (size_t)q * n + g);
+HD T ldq(const double *v, const double *d, int q, Pl n, int g) {
+  return Fld<T>::ld(v, d, ix(q, n, g));
 }
 
 // Loads of data that no thread of the running kernel writes (or that only
@@ -143,7 +158,7 @@ HD X rd(const X *p) {
   return *p;
 #endif
 }
-HD double ldr(const double *p, int q, int n, int g) { return rd(p + (size_t)q * n + g); }
+HD double ldr(const double *p, int q, Pl n, int g) { return rd(p + ix(q, n, g)); }
 
 // Starts moving the line holding *p into L2 without waiting for it (no
 // register, no effect on results): the later load of the same line then
@@ -151,9 +166,9 @@ HD double ldr(const double *p, int q, int n, int g) { return rd(p + (size_t)q * 
 __device__ __forceinline__ void pf(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
-// The same for the n-plane SoA value of cell g in each plane.
-__device__ __forceinline__ void pf_planes(const double *p, int planes, int n, int g) {
-  for (int q = 0; q < planes; ++q) pf(p + (size_t)q * n + g);
+// The same for the first `planes` planes of cell g of an n-plane array.
+__device__ __forceinline__ void pf_planes(const double *p, int planes, Pl n, int g) {
+  for (int q = 0; q < planes; ++q) pf(p + ix(q, n, g));
 }
 template <typename T> struct FldR;
 template <> struct FldR<double> {
@@ -163,12 +178,56 @@ template <> struct FldR<Dual> {
   static HD Dual ld(const double *v, const double *d, size_t i) { return Dual(rd(v + i), rd(d + i)); }
 };
 template <typename T>
-HD T ldqr(const double *v, const double *d, int q, int n, int g) {
-  return FldR<T>::ld(v, d, (size_t)q * n + g);
+HD T ldqr(const double *v, const double *d, int q, Pl n, int g) {
+  return FldR<T>::ld(v, d, ix(q, n, g));
 }
 template <typename T>
-HD void stq(double *v, double *d, int q, int n, int g, const T &x) {
-  Fld<T>::st(v, d, (size_t)q * n + g, x);
+HD void stq(double *v, double *d, int q, Pl n, int g, const T &x) {
+  Fld<T>::st(v, d, ix(q, n, g), x);
+}
+
+// K planes from plane q0 of cell g.  NC: through the read-only path (see rd).
+template <int K, bool NC>
+HD void ldk(const double *v, int q0, Pl n, int g, double *x) {
+  const double *p = v + ix(q0, n, g);
+#pragma unroll
+  for (int k = 0; k < K; ++k) x[k] = NC ? rd(p + 32 * k) : p[32 * k];
+}
+template <int K, typename T, bool NC = false>
+HD void ldk(const double *v, const double *d, int q0, Pl n, int g, T *x) {
+  double a[K];
+  ldk<K, NC>(v, q0, n, g, a);
+  if constexpr (std::is_same<T, Dual>::value) {
+    double b[K];
+    ldk<K, NC>(d, q0, n, g, b);
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = Dual(a[k], b[k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = a[k];
+  }
+}
+// and their store
+template <int K>
+HD void stk(double *v, int q0, Pl n, int g, const double *x) {
+  double *p = v + ix(q0, n, g);
+#pragma unroll
+  for (int k = 0; k < K; ++k) p[32 * k] = x[k];
+}
+template <int K, typename T>
+HD void stk(double *v, double *d, int q0, Pl n, int g, const T *x) {
+  if constexpr (std::is_same<T, Dual>::value) {
+    double a[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      a[k] = x[k].v;
+      b[k] = x[k].d;
+    }
+    stk<K>(v, q0, n, g, a);
+    stk<K>(d, q0, n, g, b);
+  } else {
+    stk<K>(v, q0, n, g, x);
+  }
 }
 
 // ---------------------------------------------------------------------------

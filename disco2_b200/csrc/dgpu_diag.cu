@@ -29,7 +29,6 @@ __global__ void __launch_bounds__(DIAG_BLK) k_diag_annulus(DevPtrs d, int inst, 
   const InstState &S = d.ist[inst];
   const int a = P.ann_base + blockIdx.x;
   const Annulus &A = d.ann[a];
-  const int N = d.n_cells;
   double acc[DIAG_NROW];
 #pragma unroll
   for (int n = 0; n < DIAG_NROW; ++n) acc[n] = 0.0;
@@ -46,12 +45,12 @@ __global__ void __launch_bounds__(DIAG_BLK) k_diag_annulus(DevPtrs d, int inst, 
       const int g = A.cell_off + j;
       const double dphi = d.dphi[g];
       const double phi = d.tiph0[g] - 0.5 * dphi;
-      const double rho = ld(d.prim, D_RHO, N, g);
-      const double press = ld(d.prim, D_PPP, N, g);
-      const double vr = ld(d.prim, D_URR, N, g);
-      const double vp_minus_w = ld(d.prim, D_UPP, N, g) * r;
-      const double vp = ld(d.prim, D_UPP, N, g) * r + rom;
-      const double vz = ld(d.prim, D_UZZ, N, g);
+      const double rho = ld(d.prim, D_RHO, Pl{d.qs}, g);
+      const double press = ld(d.prim, D_PPP, Pl{d.qs}, g);
+      const double vr = ld(d.prim, D_URR, Pl{d.qs}, g);
+      const double vp_minus_w = ld(d.prim, D_UPP, Pl{d.qs}, g) * r;
+      const double vp = ld(d.prim, D_UPP, Pl{d.qs}, g) * r + rom;
+      const double vz = ld(d.prim, D_UZZ, Pl{d.qs}, g);
       const double v2 = vr * vr + vp * vp + vz * vz;
       const double rhoe = press / (P.gamma - 1.);
       const double KE = 0.5 * rho * v2;
@@ -59,7 +58,7 @@ __global__ void __launch_bounds__(DIAG_BLK) k_diag_annulus(DevPtrs d, int inst, 
       const double dV = 0.5 * (rp * rp - rm * rm) * dphi;
       // cells with no cooling keep Cool = 0; the passive column is prim[NUM_C]
       // (with NUM_Q = 5 the reference reads past prim[] there; zero here)
-      const double cool = 0.0, passive = P.num_n > 0 ? ld(d.prim, 5, N, g) : 0.0;
+      const double cool = 0.0, passive = P.num_n > 0 ? ld(d.prim, 5, Pl{d.qs}, g) : 0.0;
       const double col[DIAG_NVEC] = {r, rho, press, vr, vp, vz, vp_minus_w, cool, passive, E_hydro, KE, rhoe,
                                      0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -147,11 +146,10 @@ __global__ void __launch_bounds__(BLK) k_diag_finish(DevPtrs d, int inst, const 
     {
       const Annulus &A0 = d.ann[P.ann_base];
       const int npw = imax < NR ? d.ann[P.ann_base + imax].np : 0;
-      const int N = d.n_cells;
       for (int j = 0; j < npw && j < P.n_cells; ++j) {
         const int g = P.cell_base + j;
         const double dV = 0.5 * (A0.rp * A0.rp - A0.rm * A0.rm) * d.dphi[g];
-        wedge += ld(d.prim, D_RHO, N, g) * dV;
+        wedge += ld(d.prim, D_RHO, Pl{d.qs}, g) * dV;
       }
     }
     extra[0] = mdot;

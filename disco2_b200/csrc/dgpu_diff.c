@@ -35,7 +35,7 @@
 
 /* A stored state: every per-cell array a substep reads, and the disk state. */
 typedef struct {
-  double *buf; /* [19][n_cells]: prim, cons, rkcons (5 each), tiph0, tiph1, rktiph, dphi */
+  double *buf; /* prim, cons, rkcons (qs planes of n_pad cells each), tiph0, tiph1, rktiph, dphi */
   InstState *ist;
 } Snap;
 
@@ -66,7 +66,7 @@ struct dgpu_diff {
   int n_snaps;
   double **tab_buf[2];
   InstState **tab_ist[2];
-  double *rec[2]; /* per set [2K][6][n_cells]: conserved sums and new widths of the substeps */
+  double *rec[2]; /* per set [2K][6 planes, n_pad cells]: conserved sums and new widths of the substeps */
   int tab_K, tab_base;
   /* the replay's own copy of the per-cell and per-face buffers (tables shared) */
   DevPtrs sh;
@@ -185,11 +185,13 @@ static int ensure_obj(struct dgpu_ctx *c, struct dgpu_diff *D, int nsteps) {
   return DGPU_OK;
 }
 
+/* doubles of the tangent arrays: 5 state arrays of 5 planes, fS, fphi, src, frf */
+#define TAN_DOUBLES(N, S) (25 * (N) + 5 * (S) + 16 * (N) + 8 * (S))
 static int ensure_tan(struct dgpu_ctx *c, struct dgpu_diff *D) {
-  size_t N = (size_t)c->n_cells, S = (size_t)(c->n_slots ? c->n_slots : 1), n;
+  size_t N = DGPU_PAD(c->n_cells), S = DGPU_PAD(c->n_slots ? c->n_slots : 1), n;
   double *p;
   if (D->t_buf) return DGPU_OK;
-  n = 25 * N + 5 * S + 16 * N + 8 * S;
+  n = TAN_DOUBLES(N, S);
   CK(cudaMalloc((void **)&D->t_buf, sizeof(double) * n));
   CK(cudaMalloc((void **)&D->t_seed, sizeof(double) * DGPU_TP_N));
   p = D->t_buf;
@@ -207,7 +209,7 @@ static int ensure_tan(struct dgpu_ctx *c, struct dgpu_diff *D) {
 }
 
 static int ensure_adj(struct dgpu_ctx *c, struct dgpu_diff *D) {
-  size_t N = (size_t)c->n_cells, S = (size_t)(c->n_slots ? c->n_slots : 1), rows, n;
+  size_t N = DGPU_PAD(c->n_cells), S = DGPU_PAD(c->n_slots ? c->n_slots : 1), rows, n;
   double *p;
   if (D->j_buf) return DGPU_OK;
   rows = (size_t)dgk_adj_rows(&c->d) + 1;
@@ -246,7 +248,7 @@ static int ensure_snaps(struct dgpu_ctx *c, struct dgpu_diff *D, int nck, int K)
     for (k = D->n_snaps; k < count; ++k) {
       D->snaps[k].buf = NULL;
       D->snaps[k].ist = NULL;
-      if (cudaMalloc((void **)&D->snaps[k].buf, sizeof(double) * 19 * (size_t)c->n_cells) != cudaSuccess ||
+      if (cudaMalloc((void **)&D->snaps[k].buf, sizeof(double) * (3 * (size_t)c->d.qs * (size_t)c->d.n_pad + 4 * (size_t)c->n_cells)) != cudaSuccess ||
           cudaMalloc((void **)&D->snaps[k].ist, sizeof(InstState) * (size_t)c->n_inst) != cudaSuccess) {
         cudaFree(D->snaps[k].buf);
         D->n_snaps = k;
@@ -278,7 +280,7 @@ static int ensure_snaps(struct dgpu_ctx *c, struct dgpu_diff *D, int nck, int K)
       D->tab_buf[set] = NULL;
       D->tab_ist[set] = NULL;
       D->rec[set] = NULL;
-      if (cudaMalloc((void **)&D->rec[set], sizeof(double) * 12 * (size_t)K * (size_t)c->n_cells) != cudaSuccess ||
+      if (cudaMalloc((void **)&D->rec[set], sizeof(double) * 12 * (size_t)K * (size_t)c->d.n_pad) != cudaSuccess ||
           cudaMalloc((void **)&D->tab_buf[set], sizeof(double *) * (size_t)(2 * K + 1)) != cudaSuccess ||
           cudaMalloc((void **)&D->tab_ist[set], sizeof(InstState *) * (size_t)(2 * K + 1)) != cudaSuccess ||
           cudaMemcpy(D->tab_buf[set], hb, sizeof(double *) * (size_t)(2 * K + 1), cudaMemcpyHostToDevice) !=
@@ -306,7 +308,7 @@ static int ensure_snaps(struct dgpu_ctx *c, struct dgpu_diff *D, int nck, int K)
 /* Lays out in fresh device memory (*mem) a copy of every per-cell, per-face
  * and per-disk buffer the step writes, in *h; the tables stay shared. */
 static int alloc_shadow(struct dgpu_ctx *c, DevPtrs *h, void **mem) {
-  const size_t N = (size_t)c->n_cells, S = (size_t)(c->n_slots ? c->n_slots : 1), A = (size_t)c->n_ann;
+  const size_t N = DGPU_PAD(c->n_cells), S = DGPU_PAD(c->n_slots ? c->n_slots : 1), A = (size_t)c->n_ann;
   const size_t R = (size_t)(c->n_runs ? c->n_runs : 1), B = (size_t)c->n_upd_blocks;
   size_t sz[32], off[33], k = 0, n;
   char *m;
@@ -617,13 +619,13 @@ int dgpu_tangent(dgpu_ctx *c, int nsteps, int window_start, double dq_dir, doubl
   seed[DGPU_TP_DALPHA] = dalpha_dir;
   CK(cudaMemcpyAsync(D->t_seed, seed, sizeof(seed), cudaMemcpyHostToDevice, c->stream));
   {
-    size_t N = (size_t)c->n_cells, S = (size_t)(c->n_slots ? c->n_slots : 1);
-    CK(cudaMemsetAsync(D->t_buf, 0, sizeof(double) * (41 * N + 13 * S), c->stream));
+    size_t N = DGPU_PAD(c->n_cells), S = DGPU_PAD(c->n_slots ? c->n_slots : 1);
+    CK(cudaMemsetAsync(D->t_buf, 0, sizeof(double) * TAN_DOUBLES(N, S), c->stream));
   }
   if (dprim) {
     CK(cudaMemcpyAsync(c->d_stage, dprim, sizeof(double) * 5 * (size_t)c->n_cells, cudaMemcpyHostToDevice,
                        c->stream));
-    CKK(dgk_aos_to_soa(D->t.prim, 5, c->n_cells, 0, c->d_stage, c->n_cells, c->stream));
+    CKK(dgk_aos_to_soa(D->t.prim, 5, c->d.qs, 0, c->d_stage, c->n_cells, c->stream));
   }
   CKK(dgk_calc_cons(&c->d, &D->t, c->stream));
   CKK(dgk_set_int(D->d_idx, 0, c->stream));
@@ -690,7 +692,7 @@ int dgpu_adjoint(dgpu_ctx *c, int nsteps, int window_start, int ckpt_every, cons
   /* reverse sweep, segment by segment: the replay of segment seg - 1 (shadow
    * buffers, stream s2, stored-state set (seg - 1) % 2) runs while segment seg
    * is reversed (context buffers, the context's stream, set seg % 2) */
-  CK(cudaMemsetAsync(D->J.lW, 0, sizeof(double) * 15 * N, c->stream));
+  CK(cudaMemsetAsync(D->J.lW, 0, sizeof(double) * 15 * (size_t)c->d.n_pad, c->stream));
   CK(cudaMemsetAsync(D->J.acc, 0, sizeof(double) * 8, c->stream));
   CK(cudaEventRecord(D->e_rev, c->stream));
   for (seg = nck; seg >= 0; --seg) {
@@ -723,7 +725,7 @@ int dgpu_adjoint(dgpu_ctx *c, int nsteps, int window_start, int ckpt_every, cons
   CKK(dgk_snap(&c->d, ck[0].buf, ck[0].ist, 0, c->stream));
   CKK(dgk_adj_calc_cons(&c->d, &D->J, c->stream));
   if (dJ_dprim) {
-    CKK(dgk_soa_to_aos(c->d_stage, 5, c->n_cells, 0, D->J.lW, c->n_cells, c->stream));
+    CKK(dgk_soa_to_aos(c->d_stage, 5, 5, 0, D->J.lW, c->n_cells, c->stream));
     CK(cudaMemcpyAsync(dJ_dprim, c->d_stage, sizeof(double) * 5 * N, cudaMemcpyDeviceToHost, c->stream));
   }
   CK(cudaMemcpyAsync(acc, D->J.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream));

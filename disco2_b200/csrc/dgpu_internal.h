@@ -3,8 +3,9 @@
  *
  * Cells of every disk in a context are numbered globally, disk after disk,
  * each disk in the reference's (k, i, j) order (annulus-major: annulus i holds
- * N_p[i] consecutive cells).  Per-cell variables are structure-of-arrays:
- * variable q of cell g lives at X[q * n_cells + g].  Annulus-level constants
+ * N_p[i] consecutive cells).  Variables of several planes per cell or face are
+ * in tiles of 32 cells, plane after plane (ix in dgpu_device.cuh), below as
+ * [planes][cells]; single ones are plain arrays.  Annulus-level constants
  * (radii, frame terms, boundary profile) live in an Annulus table; the r-faces
  * of the annulus pair (i, i+1) of a disk live in a slab of capacity
  * N_p[i] + N_p[i+1] + DGPU_FACE_SLACK starting at Annulus.face_base.
@@ -15,6 +16,8 @@
 #include <stdint.h>
 
 #define DGPU_NQ 5
+#define DGPU_TILE 32        /* cells of a tile of the several-plane arrays */
+#define DGPU_PAD(n) (((size_t)(n) + DGPU_TILE - 1) / DGPU_TILE * DGPU_TILE)
 #define DGPU_MAX_PASSIVE 3  /* NUM_N at most */
 #define DGPU_FACE_SLACK 8
 #define DGPU_RUN_SLACK 8
@@ -147,6 +150,8 @@ typedef struct {
 /* Device pointers and sizes handed to every kernel. */
 typedef struct {
   int n_inst, n_ann, n_cells, n_slots, n_runs;
+  int n_pad;              /* n_cells rounded up to whole tiles of 32 */
+  int qs, qf;             /* planes of the state arrays (5 + n_pass) and of fphi and frf (8 + n_pass) */
   const DiskParams *par;
   InstState *ist;
   const Annulus *ann;
@@ -312,8 +317,8 @@ int dgk_diagnostics(const DevPtrs *d, int inst, int n_ann_disk, double *rows, do
 int dgk_torque(const DevPtrs *d, int inst, double *part, double *out, int n_inst_cells, void *stream);
 int dgk_update_blocks(int n_cells);
 int dgk_block_size(void);
-int dgk_aos_to_soa(double *soa, int nq, int stride, int base, const double *aos, int n, void *stream);
-int dgk_soa_to_aos(double *aos, int nq, int stride, int base, const double *soa, int n, void *stream);
+int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, void *stream);
+int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream);
 #ifdef __cplusplus
 }
 #endif

@@ -44,6 +44,9 @@
 #ifndef DGPU_MINB_FACE
 #define DGPU_MINB_FACE 6
 #endif
+#ifndef DGPU_MINB_CELLPREP
+#define DGPU_MINB_CELLPREP 5
+#endif
 #ifndef DGPU_MINB_PLM
 #define DGPU_MINB_PLM 4
 #endif
@@ -179,9 +182,9 @@ __device__ T block_excl_scan(T v, T *sh, T &total) {
 // (src/Cell/cell_misc.c:12-26) and cell_plm_p (src/Cell/cell_plm.c:116-161).
 template <typename T, bool PS>
 __device__ __forceinline__ void cellprep_cell(const DevPtrs &d, const TanPtrs &tp, int g, int substep) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5};
   const double *traw = substep == 1 ? d.tiph0 : d.tiph1;
-  pf_planes(d.prim, 5, N, g);
+  pf_planes(d.prim, 5, QS, g);
   pf(d.dphi + g);
   pf(traw + g);
   const int a = d.cell_ann[g];
@@ -194,21 +197,30 @@ __device__ __forceinline__ void cellprep_cell(const DevPtrs &d, const TanPtrs &t
   const double dc = d.dphi[g];
   const double dpL = .5 * (dc + d.dphi[gl]);
   const double dpR = .5 * (dc + d.dphi[gr]);
+  const double plm = P.plm;
+  // two planes at a time: all five at once spill at this kernel's registers
+  auto slopes = [&](auto K, int q) {
+    T pc[2], pl[2], pr[2];
+    ldk<K.value, T, true>(d.prim, tp.prim, q, QS, g, pc);
+    ldk<K.value, T, true>(d.prim, tp.prim, q, QS, gl, pl);
+    ldk<K.value, T, true>(d.prim, tp.prim, q, QS, gr, pr);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    T pc = ldq<T>(d.prim, tp.prim, q, N, g), pl = ldq<T>(d.prim, tp.prim, q, N, gl),
-      pr = ldq<T>(d.prim, tp.prim, q, N, gr);
-    stq<T>(d.gradp, tp.gradp, q, N, g, plm_p_slope(pl, pc, pr, dpL, dpR, P.plm));
-  }
+    for (int k = 0; k < K.value; ++k) pc[k] = plm_p_slope(pl[k], pc[k], pr[k], dpL, dpR, plm);
+    stk<K.value, T>(d.gradp, tp.gradp, q, QS, g, pc);
+  };
+  slopes(std::integral_constant<int, 2>(), 0);
+  slopes(std::integral_constant<int, 2>(), 2);
+  slopes(std::integral_constant<int, 1>(), 4);
   for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q)
-    d.gradp[(size_t)q * N + g] = plm_p_slope(ld(d.prim, q, N, gl), ld(d.prim, q, N, g), ld(d.prim, q, N, gr), dpL, dpR, P.plm);
+    d.gradp[ix(q, QS, g)] =
+        plm_p_slope(ld(d.prim, q, QS, gl), ld(d.prim, q, QS, g), ld(d.prim, q, QS, gr), dpL, dpR, P.plm);
 }
 
 // cellprep_cell for every cell and, for the first cell of each disk,
 // gravMass_copy at the start of a step (GravMass_misc.c:20-28) and
 // gravMass_clean_pi (GravMass_misc.c:9-17).  Runs concurrently with k_merge.
 template <typename T, bool PS = false>
-__global__ void __launch_bounds__(BLK, DGPU_MINB_FACE) k_cellprep(DevPtrs d, TanPtrs tp, int substep) {
+__global__ void __launch_bounds__(BLK, DGPU_MINB_CELLPREP) k_cellprep(DevPtrs d, TanPtrs tp, int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.n_cells) return;
   cellprep_cell<T, PS>(d, tp, g, substep);
@@ -268,7 +280,7 @@ __device__ __forceinline__ void merge_pair(const DevPtrs &d, int a, int substep)
   const double *traw = substep == 1 ? d.tiph0 : d.tiph1;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int np = A.np, off = A.cell_off;
-  const int N = d.n_cells;
+  const Pl QS = {d.qs};
   const bool rigid = P.w_numeric == DC_RIGID;
   if (!Z && tid == 0 && !rigid) d.w_ann[a] = A.wnum;
   if (!Z && tid >= nt - 32 && P.w_analytic == DA_MILOS) milos_frame(d, P, A, a, tid & 31);
@@ -487,8 +499,8 @@ __device__ __forceinline__ void merge_pair(const DevPtrs &d, int a, int substep)
     double w = 0.0, Mring = 0.0, x = 0.0, m = 0.0;
     auto fetch = [&](int j, double &xj, double &mj) {
       if (j >= np) return;
-      const double vp = A.r * ldr(d.prim, D_UPP, N, off + j);
-      mj = ldr(d.cons, D_DDD, N, off + j);
+      const double vp = A.r * ldr(d.prim, D_UPP, QS, off + j);
+      mj = ldr(d.cons, D_DDD, QS, off + j);
       xj = vp * mj;
     };
     fetch(lane, x, m);
@@ -535,13 +547,13 @@ __device__ __forceinline__ void rslope_face(const DevPtrs &d, const TanPtrs &tp,
   const int cL = rd(d.fL + slot);
   if (cL < 0) return;  // slot past the face list of its pair
   const int cR = rd(d.fR + slot);
-  pf_planes(d.prim, 5, d.n_cells, cL);
-  pf_planes(d.prim, 5, d.n_cells, cR);
-  pf_planes(d.gradp, 5, d.n_cells, cL);
-  pf_planes(d.gradp, 5, d.n_cells, cR);
+  const Pl QS = {PS ? d.qs : 5};
+  pf_planes(d.prim, 5, QS, cL);
+  pf_planes(d.prim, 5, QS, cR);
+  pf_planes(d.gradp, 5, QS, cL);
+  pf_planes(d.gradp, 5, QS, cR);
   const int a = rd(d.slot_ann + slot);
   const Annulus &A = d.ann[a];
-  const int N = d.n_cells, NS = d.n_slots;
   const double cm = rd(d.fcm + slot);
   double pL = rd(d.tiphw + cL) - .5 * rd(d.dphi + cL);
   double pR = rd(d.tiphw + cR) - .5 * rd(d.dphi + cR);
@@ -549,19 +561,19 @@ __device__ __forceinline__ void rslope_face(const DevPtrs &d, const TanPtrs &tp,
   dpL = wrap_pm(dpL, d.err);
   double dpR = pR - cm;
   dpR = wrap_pm(dpR, d.err);
-  d.fdp[slot] = dpL;
-  d.fdp[(size_t)NS + slot] = dpR;
+  const double dp[2] = {dpL, dpR};
+  stk<2>(d.fdp, 0, P2, slot, dp);
   const double den = A.f_dr + A.f_dl;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    T WL = ldqr<T>(d.prim, tp.prim, q, N, cL) + dpL * ldqr<T>(d.gradp, tp.gradp, q, N, cL);
-    T WR = ldqr<T>(d.prim, tp.prim, q, N, cR) - dpR * ldqr<T>(d.gradp, tp.gradp, q, N, cR);
-    stq<T>(d.fS, tp.fS, q, NS, slot, (WR - WL) / den);
+    const T WL = ldqr<T>(d.prim, tp.prim, q, QS, cL) + dpL * ldqr<T>(d.gradp, tp.gradp, q, QS, cL);
+    const T WR = ldqr<T>(d.prim, tp.prim, q, QS, cR) - dpR * ldqr<T>(d.gradp, tp.gradp, q, QS, cR);
+    stq<T>(d.fS, tp.fS, q, QS, slot, (WR - WL) / den);
   }
   for (int q = 5; q < 5 + (PS ? d.par[A.inst].num_n : 0); ++q) {
-    const double WL = ldr(d.prim, q, N, cL) + dpL * ldr(d.gradp, q, N, cL);
-    const double WR = ldr(d.prim, q, N, cR) - dpR * ldr(d.gradp, q, N, cR);
-    d.fS[(size_t)q * NS + slot] = (WR - WL) / den;
+    const double WL = ldr(d.prim, q, QS, cL) + dpL * ldr(d.gradp, q, QS, cL);
+    const double WR = ldr(d.prim, q, QS, cR) - dpR * ldr(d.gradp, q, QS, cR);
+    d.fS[ix(q, QS, slot)] = (WR - WL) / den;
   }
 }
 
@@ -579,15 +591,16 @@ template <typename T>
 __device__ __noinline__ void limit_seq(const DevPtrs &d, const TanPtrs &tp, int g, int q) {
   const int a = d.cell_ann[g];
   const DiskParams &P = d.par[d.ann[a].inst];
-  T gq = ldq<T>(d.grad, tp.grad, q, d.n_cells, g);
+  const Pl QS = {d.qs};
+  T gq = ldq<T>(d.grad, tp.grad, q, QS, g);
   for_cell_rface_ranges(d, d.ann[a], a, g, P.NR, [&](int s, int e, int) {
     for (int n = s; n < e; ++n) {
-      const T S = ldq<T>(d.fS, tp.fS, q, d.n_slots, n);
+      const T S = ldq<T>(d.fS, tp.fS, q, QS, n);
       if (S * gq < 0.0) gq = 0.0;
       else if (fabs(P.plm * S) < fabs(gq)) gq = P.plm * S;
     }
   });
-  stq<T>(d.grad, tp.grad, q, d.n_cells, g, gq);
+  stq<T>(d.grad, tp.grad, q, QS, g, gq);
 }
 
 // cell_plm_rz's r slope of cell g (src/Cell/cell_plm.c:56-114): the
@@ -606,7 +619,7 @@ __device__ __noinline__ void limit_seq(const DevPtrs &d, const TanPtrs &tp, int 
 // face-parallel kernel has no such waste.
 template <typename T, bool PS>
 __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, int g) {
-  const int N = d.n_cells, NS = d.n_slots;
+  const Pl QS = {PS ? d.qs : 5};
   pf(d.rr + 4 * (size_t)g);
   pf(d.fstart + g);
   pf(d.dphi + g);
@@ -626,9 +639,11 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
     const double fr = Q.f_r, fperp = Q.f_dperp;
     for (int n = s; n < e; ++n) {
       const double dA = fr * rd(d.fdphi + n) * fperp;
+      T Sf[5];
+      ldk<5, T>(d.fS, tp.fS, 0, QS, n, Sf);
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        const T S = ldq<T>(d.fS, tp.fS, q, NS, n);
+        const T S = Sf[q];
         gq[q] += S * dA;
         const T ps = plm * S;
         if (fabs(ps) < fabs(lim[q])) lim[q] = ps;
@@ -655,17 +670,18 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
     } else if (fabs(lim[q]) < fabs(m)) {
       m = lim[q];
     }
-    stq<T>(d.grad, tp.grad, q, N, g, m);
+    gq[q] = m;
   }
+  stk<5, T>(d.grad, tp.grad, 0, QS, g, gq);
   for (; seq; seq &= seq - 1) limit_seq<T>(d, tp, g, __ffs(seq) - 1);
   // passive scalars: the same face-weighted slope and limiter
   for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q) {
     double gs = 0.0;
     for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int) {
       double dA = F.r * F.dphi * F.dperp;
-      gs += ld(d.fS, q, NS, slot) * dA;
+      gs += ld(d.fS, q, QS, slot) * dA;
     });
-    d.grad[(size_t)q * N + g] = gs / dAtot;
+    d.grad[ix(q, QS, g)] = gs / dAtot;
     limit_seq<double>(d, tp, g, q);
   }
 }
@@ -677,7 +693,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
 __device__ __forceinline__ unsigned long long cfl_key(const DevPtrs &d, const Annulus &A, const DiskParams &P,
                                                       int g, double wa, const double *rkx, const double *rky,
                                                       const double *rkM) {
-  const int N = d.n_cells;
+  const Pl QS = {d.qs};
   const double *traw = d.tiph0;
   double w = .5 * (wa + wa);
   double dr = A.rp - A.rm;
@@ -686,9 +702,9 @@ __device__ __forceinline__ unsigned long long cfl_key(const DevPtrs &d, const An
   double rdphi = .5 * (A.rp + A.rm) * d.dphi[g];
   if (rdphi < dr) dx = rdphi;
   if (dx > A.dz) dx = A.dz;
-  double Pp = ld(d.prim, D_PPP, N, g), rho = ld(d.prim, D_RHO, N, g);
-  double vp = ld(d.prim, D_UPP, N, g) * r - w;
-  double vr = ld(d.prim, D_URR, N, g), vz = ld(d.prim, D_UZZ, N, g);
+  double Pp = ld(d.prim, D_PPP, QS, g), rho = ld(d.prim, D_RHO, QS, g);
+  double vp = ld(d.prim, D_UPP, QS, g) * r - w;
+  double vr = ld(d.prim, D_URR, QS, g), vz = ld(d.prim, D_UZZ, QS, g);
   double cs = sqrt(P.gamma * Pp / rho);
   double cf2 = cs * cs;
   double maxv = sqrt(cf2) + sqrt(vr * vr + vp * vp + vz * vz);
@@ -787,12 +803,12 @@ __global__ void k_dt(DevPtrs d) {
 template <typename T, bool PS>
 __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &tp, int g, const InstState *ist,
                                               int substep) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   // the cell's own planes (its right neighbour's share the lines) ahead of
   // the annulus lookups
-  pf_planes(d.prim, 5, N, g);
-  pf_planes(d.gradp, 5, N, g);
-  pf_planes(d.grad, 5, N, g);
+  pf_planes(d.prim, 5, QS, g);
+  pf_planes(d.gradp, 5, QS, g);
+  pf_planes(d.grad, 5, QS, g);
   pf(d.tiphw + g);
   pf(d.dphi + g);
   const int a = d.cell_ann[g];
@@ -806,34 +822,39 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
   const double r = .5 * (A.rp + A.rm);
   const double dA = dr * dz;
   T pL[5], pR[5];
+  {
+    T gL[5], gR[5];
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, pL);
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, pR);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, gL);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, gR);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    pL[q] = ldq<T>(d.prim, tp.prim, q, N, cL) + 0.5 * ldq<T>(d.gradp, tp.gradp, q, N, cL) * dpL;
-    pR[q] = ldq<T>(d.prim, tp.prim, q, N, cR) - 0.5 * ldq<T>(d.gradp, tp.gradp, q, N, cR) * dpR;
+    for (int q = 0; q < 5; ++q) {
+      pL[q] = pL[q] + 0.5 * gL[q] * dpL;
+      pR[q] = pR[q] - 0.5 * gR[q] * dpR;
+    }
   }
   const double w = d.w_ann[a];
   T F[5];
   double qL[DGPU_MAX_PASSIVE], qR[DGPU_MAX_PASSIVE], Fq[DGPU_MAX_PASSIVE];
   const int np = PS ? P.num_n : 0;
   for (int s = 0; s < np; ++s) {
-    qL[s] = ld(d.prim, 5 + s, N, cL) + 0.5 * ld(d.gradp, 5 + s, N, cL) * dpL;
-    qR[s] = ld(d.prim, 5 + s, N, cR) - 0.5 * ld(d.gradp, 5 + s, N, cR) * dpR;
+    qL[s] = ld(d.prim, 5 + s, QS, cL) + 0.5 * ld(d.gradp, 5 + s, QS, cL) * dpL;
+    qR[s] = ld(d.prim, 5 + s, QS, cR) - 0.5 * ld(d.gradp, 5 + s, QS, cR) * dpR;
   }
   riemann_flux(pL, pR, r, 1, w, P.gamma, P.riemann, F, np, qL, qR, Fq);
   const InstState &S = ist ? *ist : d.ist[A.inst];
   const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) stq<T>(d.fphi, tp.fphi, q, N, g, k * F[q]);
-  for (int s = 0; s < np; ++s) d.fphi[(size_t)(8 + s) * N + g] = k * Fq[s];
+  for (int q = 0; q < 5; ++q) F[q] = k * F[q];
+  stk<5, T>(d.fphi, tp.fphi, 0, QF, g, F);
+  for (int s = 0; s < np; ++s) d.fphi[ix(8 + s, QF, g)] = k * Fq[s];
   if (P.has_visc) {
     ViscIn<T> v;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      v.cL[q] = ldq<T>(d.prim, tp.prim, q, N, cL);
-      v.cR[q] = ldq<T>(d.prim, tp.prim, q, N, cR);
-      v.grL[q] = ldq<T>(d.grad, tp.grad, q, N, cL);
-      v.grR[q] = ldq<T>(d.grad, tp.grad, q, N, cR);
-    }
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
+    ldk<4, T>(d.grad, tp.grad, 0, QS, cL, v.grL);
+    ldk<4, T>(d.grad, tp.grad, 0, QS, cR, v.grR);
     v.tL = d.tiphw[cL];
     v.tR = d.tiphw[cR];
     v.dpL = v.dpR = 0.0;
@@ -844,10 +865,11 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
     v.rdr_om = frame_val(d, P, A.rdrom, a, DGPU_FR_RDROM);
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
-    T Fv[3];
+    T Fv[3], u[4];
     visc_flux(v, 1, P, G, Fv, d.err);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) stq<T>(d.fphi, tp.fphi, 5 + q, N, g, k * Fv[q]);
+    for (int q = 0; q < 3; ++q) u[1 + q] = k * Fv[q];
+    stk<3, T>(d.fphi, tp.fphi, 5, QF, g, u + 1);
   }
 }
 
@@ -862,7 +884,7 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_flux_phi(DevPtrs d,
 template <typename T, bool PS>
 __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp, int slot, const InstState *ist,
                                             int substep) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   const int cL = d.fL[slot];
   if (cL < 0) return;  // slot past the face list of its pair
   const int cR = d.fR[slot];
@@ -871,43 +893,47 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
   const DiskParams &P = d.par[A.inst];
   const double fdphi = d.fdphi[slot], cm = d.fcm[slot];
   const double deltaL = A.f_dl, deltaR = A.f_dr;
-  const double dpL = d.fdp[slot];
-  const double dpR = d.fdp[(size_t)d.n_slots + slot];
+  double dp[2];
+  ldk<2, false>(d.fdp, 0, P2, slot, dp);
+  const double dpL = dp[0], dpR = dp[1];
   const double r = A.f_r;
   const double dA = r * fdphi * A.f_dperp;
   const double r_cell_L = r - deltaL;
   const double r_cell_R = r + deltaR;
   T pL[5], pR[5];
+  {
+    T u[5], w[5];
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, pL);
+    ldk<5, T>(d.grad, tp.grad, 0, QS, cL, u);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, w);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    pL[q] = ldq<T>(d.prim, tp.prim, q, N, cL) + ldq<T>(d.grad, tp.grad, q, N, cL) * deltaL +
-            ldq<T>(d.gradp, tp.gradp, q, N, cL) * dpL;
-    pR[q] = ldq<T>(d.prim, tp.prim, q, N, cR) - ldq<T>(d.grad, tp.grad, q, N, cR) * deltaR -
-            ldq<T>(d.gradp, tp.gradp, q, N, cR) * dpR;
+    for (int q = 0; q < 5; ++q) pL[q] = pL[q] + u[q] * deltaL + w[q] * dpL;
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, pR);
+    ldk<5, T>(d.grad, tp.grad, 0, QS, cR, u);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, w);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) pR[q] = pR[q] - u[q] * deltaR - w[q] * dpR;
   }
   T F[5];
   double qL[DGPU_MAX_PASSIVE], qR[DGPU_MAX_PASSIVE], Fq[DGPU_MAX_PASSIVE];
   const int np = PS ? P.num_n : 0;
   for (int s = 0; s < np; ++s) {
-    qL[s] = ld(d.prim, 5 + s, N, cL) + ld(d.grad, 5 + s, N, cL) * deltaL + ld(d.gradp, 5 + s, N, cL) * dpL;
-    qR[s] = ld(d.prim, 5 + s, N, cR) - ld(d.grad, 5 + s, N, cR) * deltaR - ld(d.gradp, 5 + s, N, cR) * dpR;
+    qL[s] = ld(d.prim, 5 + s, QS, cL) + ld(d.grad, 5 + s, QS, cL) * deltaL + ld(d.gradp, 5 + s, QS, cL) * dpL;
+    qR[s] = ld(d.prim, 5 + s, QS, cR) - ld(d.grad, 5 + s, QS, cR) * deltaR - ld(d.gradp, 5 + s, QS, cR) * dpR;
   }
   riemann_flux(pL, pR, r, 0, 0.0, P.gamma, P.riemann, F, np, qL, qR, Fq);
   const InstState &S = ist ? *ist : d.ist[A.inst];
   const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
-  const int NS = d.n_slots;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) stq<T>(d.frf, tp.frf, q, NS, slot, k * F[q]);
-  for (int s = 0; s < np; ++s) d.frf[(size_t)(8 + s) * NS + slot] = k * Fq[s];
+  for (int q = 0; q < 5; ++q) F[q] = k * F[q];
+  stk<5, T>(d.frf, tp.frf, 0, QF, slot, F);
+  for (int s = 0; s < np; ++s) d.frf[ix(8 + s, QF, slot)] = k * Fq[s];
   if (P.has_visc) {
     ViscIn<T> v;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      v.cL[q] = ldq<T>(d.prim, tp.prim, q, N, cL);
-      v.cR[q] = ldq<T>(d.prim, tp.prim, q, N, cR);
-      v.gpL[q] = ldq<T>(d.gradp, tp.gradp, q, N, cL);
-      v.gpR[q] = ldq<T>(d.gradp, tp.gradp, q, N, cR);
-    }
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
+    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, v.gpL);
+    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, v.gpR);
     v.tL = d.tiphw[cL];
     v.tR = d.tiphw[cR];
     v.dpL = dpL;
@@ -919,10 +945,11 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
     v.rdr_om = frame_val(d, P, A.f_rdrom, a, DGPU_FR_FRDROM);
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
-    T Fv[3];
+    T Fv[3], u[4];
     visc_flux(v, 0, P, G, Fv, d.err);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) stq<T>(d.frf, tp.frf, 5 + q, NS, slot, k * Fv[q]);
+    for (int q = 0; q < 3; ++q) u[1 + q] = k * Fv[q];
+    stk<3, T>(d.frf, tp.frf, 5, QF, slot, u + 1);
   }
 }
 
@@ -948,7 +975,6 @@ __global__ void __launch_bounds__(BLK) k_zslope(DevPtrs d) {
   const int cR = rd(d.zfR + slot);
   const int a = rd(d.zslot_ann + slot);
   const Annulus &A = d.ann[a];
-  const int N = d.n_cells, NS = d.n_zslots;
   const double cm = rd(d.zfcm + slot);
   double pL = rd(d.tiphw + cL) - .5 * rd(d.dphi + cL);
   double pR = rd(d.tiphw + cR) - .5 * rd(d.dphi + cR);
@@ -956,15 +982,22 @@ __global__ void __launch_bounds__(BLK) k_zslope(DevPtrs d) {
   dpL = wrap_pm(dpL, d.err);
   double dpR = pR - cm;
   dpR = wrap_pm(dpR, d.err);
-  d.zfdp[slot] = dpL;
-  d.zfdp[(size_t)NS + slot] = dpR;
+  const double dp[2] = {dpL, dpR};
+  stk<2>(d.zfdp, 0, P2, slot, dp);
   const double den = A.zf_dr + A.zf_dl;
+  const Pl QS = {d.qs};
+  double wL[5], wR[5], gL[5], gR[5];
+  ldk<5, true>(d.prim, 0, QS, cL, wL);
+  ldk<5, true>(d.prim, 0, QS, cR, wR);
+  ldk<5, true>(d.gradp, 0, QS, cL, gL);
+  ldk<5, true>(d.gradp, 0, QS, cR, gR);
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    const double WL = ldr(d.prim, q, N, cL) + dpL * ldr(d.gradp, q, N, cL);
-    const double WR = ldr(d.prim, q, N, cR) - dpR * ldr(d.gradp, q, N, cR);
-    d.zfS[(size_t)q * NS + slot] = (WR - WL) / den;
+    const double WL = wL[q] + dpL * gL[q];
+    const double WR = wR[q] - dpR * gR[q];
+    wL[q] = (WR - WL) / den;
   }
+  stk<5>(d.zfS, 0, P5, slot, wL);
 }
 
 // cell_plm_rz with Z_DIR (src/Cell/cell_plm.c:13-114) per cell of a 3-D disk:
@@ -974,8 +1007,7 @@ __global__ void __launch_bounds__(BLK) k_zslope(DevPtrs d) {
 // fluxes and (in 3-D) the viscous source read.
 __global__ void __launch_bounds__(BLK) k_plm_z(DevPtrs d) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells, NS = d.n_zslots;
-  if (g >= N) return;
+  if (g >= d.n_cells) return;
   const int a = d.cell_ann[g];
   const Annulus &A = d.ann[a];
   const DiskParams &P = d.par[A.inst];
@@ -986,8 +1018,10 @@ __global__ void __launch_bounds__(BLK) k_plm_z(DevPtrs d) {
   for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int) {
     for (int n = s; n < e; ++n) {
       const double dA = zr * rd(d.zfdphi + n) * zperp;
+      double S[5];
+      ldk<5, true>(d.zfS, 0, P5, n, S);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) gq[q] += ld(d.zfS, q, NS, n) * dA;
+      for (int q = 0; q < 5; ++q) gq[q] += S[q] * dA;
     }
   });
   const double dp = d.dphi[g];
@@ -996,16 +1030,17 @@ __global__ void __launch_bounds__(BLK) k_plm_z(DevPtrs d) {
   for (int q = 0; q < 5; ++q) gq[q] /= dAtot;
   for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int) {
     for (int n = s; n < e; ++n) {
+      double S[5];
+      ldk<5, true>(d.zfS, 0, P5, n, S);
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        const double Sq = ld(d.zfS, q, NS, n);
+        const double Sq = S[q];
         if (Sq * gq[q] < 0.0) gq[q] = 0.0;
         else if (fabs(P.plm * Sq) < fabs(gq[q])) gq[q] = P.plm * Sq;
       }
     }
   });
-#pragma unroll
-  for (int q = 0; q < 5; ++q) d.gradz[(size_t)q * N + g] = gq[q];
+  stk<5>(d.gradz, 0, P5, g, gq);
 }
 
 // z faces: thread per face slot (riemann_setup_rz with ZDIRECTION,
@@ -1022,22 +1057,33 @@ __global__ void __launch_bounds__(BLK) k_flux_z(DevPtrs d, int substep) {
   const Annulus &A = d.ann[a];
   const DiskParams &P = d.par[A.inst];
   const InstState &S = d.ist[A.inst];
-  const int N = d.n_cells, NS = d.n_zslots;
   const double fac = substep == 1 ? 1.0 : 0.5;
   const double deltaL = A.zf_dl, deltaR = A.zf_dr;
-  const double dpL = d.zfdp[slot], dpR = d.zfdp[(size_t)NS + slot];
+  double dp[2];
+  ldk<2, true>(d.zfdp, 0, P2, slot, dp);
+  const double dpL = dp[0], dpR = dp[1];
   const double r = A.zf_r;
   const double dA = r * d.zfdphi[slot] * A.zf_dperp;
   double pL[5], pR[5], F[5];
+  {
+    const Pl QS = {d.qs};
+    double u[5], w[5];
+    ldk<5, true>(d.prim, 0, QS, cL, pL);
+    ldk<5, true>(d.gradz, 0, P5, cL, u);
+    ldk<5, true>(d.gradp, 0, QS, cL, w);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    pL[q] = ld(d.prim, q, N, cL) + ld(d.gradz, q, N, cL) * deltaL + ld(d.gradp, q, N, cL) * dpL;
-    pR[q] = ld(d.prim, q, N, cR) - ld(d.gradz, q, N, cR) * deltaR - ld(d.gradp, q, N, cR) * dpR;
+    for (int q = 0; q < 5; ++q) pL[q] = pL[q] + u[q] * deltaL + w[q] * dpL;
+    ldk<5, true>(d.prim, 0, QS, cR, pR);
+    ldk<5, true>(d.gradz, 0, P5, cR, u);
+    ldk<5, true>(d.gradp, 0, QS, cR, w);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) pR[q] = pR[q] - u[q] * deltaR - w[q] * dpR;
   }
   riemann_flux(pL, pR, r, 2, 0.0, P.gamma, P.riemann, F);
   const double k = fac * step_dt(d, S, P, substep) * dA;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) d.zfrf[(size_t)q * NS + slot] = k * F[q];
+  for (int q = 0; q < 5; ++q) F[q] = k * F[q];
+  stk<5>(d.zfrf, 0, P5, slot, F);
   if (P.has_visc) {
     // riemann_visc_flux averages the reconstructed states on a z face and
     // exits on a nonzero v_z (Riemann_routines.c:271-274)
@@ -1069,19 +1115,17 @@ __global__ void __launch_bounds__(BLK) k_zsync(DevPtrs d, int substep) {
   const Annulus &Sr = d.ann[a + (ks - A.k) * P.NR];
   const int gs = Sr.cell_off + (g - A.cell_off);
   double *tout = substep == 1 ? d.tiph1 : d.tiph0;
+  const Pl QS = {d.qs};  // (a 3-D disk itself carries no passive scalars)
   double pr[5], c[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    pr[q] = d.prim[(size_t)q * N + gs];
-    d.prim[(size_t)q * N + g] = pr[q];
-    d.rkcons[(size_t)q * N + g] = d.rkcons[(size_t)q * N + gs];
-  }
+  ldk<5, false>(d.prim, 0, QS, gs, pr);
+  stk<5>(d.prim, 0, QS, g, pr);
+  ldk<5, false>(d.rkcons, 0, QS, gs, c);
+  stk<5>(d.rkcons, 0, QS, g, c);
   tout[g] = tout[gs];
   const double r = .5 * (A.rm + A.rp);
   const double dV = A.dv_half * d.dphi[g] * A.dz;
   prim2cons(pr, c, r, dV, P.gamma);
-#pragma unroll
-  for (int q = 0; q < 5; ++q) d.cons[(size_t)q * N + g] = c[q];
+  stk<5>(d.cons, 0, QS, g, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -1126,11 +1170,11 @@ __device__ __forceinline__ void ann_consts(const DevPtrs &d, int t, const InstSt
 template <typename T, bool PS>
 __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &tp, int g, const InstState &S,
                                               double dt, double &md0, double &md1) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5};
   {
-    pf_planes(d.prim, 5, N, g);
-    pf(d.grad + (size_t)D_UPP * N + g);
-    pf(d.gradp + (size_t)D_URR * N + g);
+    pf_planes(d.prim, 5, QS, g);
+    pf(d.grad + ix(D_UPP, QS, g));
+    pf(d.gradp + ix(D_URR, QS, g));
     pf(d.tiphw + g);
     pf(d.dphi + g);
     const int a = d.cell_ann[g];
@@ -1141,8 +1185,7 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
     double phi = d.tiphw[g] - .5 * dphi;
     double r = .5 * (rp + rm);
     T pm[5];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) pm[q] = ldq<T>(d.prim, tp.prim, q, N, g);
+    ldk<5, T>(d.prim, tp.prim, 0, QS, g, pm);
     SrcGeom sg;
     sg.r = r;
     sg.dt = dt;
@@ -1173,14 +1216,12 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
     if (P.has_visc) {
       // in 3-D cell_plm_rz(Z_DIR) has overwritten grad with the z slopes by the
       // time cell_add_visc_src reads it (timestep_routines.c:63-81)
-      gu = (d.has_z && P.NZ > 1) ? T(d.gradz[(size_t)D_UPP * N + g]) : ldq<T>(d.grad, tp.grad, D_UPP, N, g);
-      gpu = ldq<T>(d.gradp, tp.gradp, D_URR, N, g);
+      gu = (d.has_z && P.NZ > 1) ? T(ld(d.gradz, D_UPP, P5, g)) : ldq<T>(d.grad, tp.grad, D_UPP, QS, g);
+      gpu = ldq<T>(d.gradp, tp.gradp, D_URR, QS, g);
     }
     T sv[6];
     source_cell(sg, P, pm, gu, gpu, G, sv);
-#pragma unroll
-    for (int q = 0; q < 5; ++q) stq<T>(d.src, tp.src, q, N, g, sv[q]);
-    if (P.has_visc) stq<T>(d.src, tp.src, 5, N, g, sv[5]);
+    stk<6, T>(d.src, tp.src, 0, P8, g, sv);
     const double xpos = sg.xpos, ypos = sg.ypos, dV = sg.dV;
     const T rho = pm[D_RHO], Pp = pm[D_PPP];
     if (P.rho_sink_on == 1) {
@@ -1202,7 +1243,7 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
         double drho = 0.0;
         if (p == 0) { if (r0 < sink_size) drho = rhov / t_visc0; }
         else { if (r1 < sink_size) drho = rhov / t_visc1; }
-        stq<T>(d.src, tp.src, 6 + p, N, g, T(drho * dt * dV));
+        stq<T>(d.src, tp.src, 6 + p, P8, g, T(drho * dt * dV));
         if (A.kind & DGPU_AK_SINK_SUM) {
           if (p == 0) md0 += drho * dV;
           else md1 += drho * dV;
@@ -1259,20 +1300,20 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
 // increments were written by other blocks of the running kernel (plain loads,
 // not the read-only path).  rec (the adjoint's segment replay, else NULL): the
 // conserved sum before cons2prim and the new width of each cell go to slot
-// 2 * (*rec_idx) + substep - 1 of rec ([slot][6][n_cells]).
+// 2 * (*rec_idx) + substep - 1 of rec (per slot 6 planes over n_pad cells).
 template <typename T, bool PS, bool XC = false>
 __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp, int g, int substep, int stop,
                                             const InstState *ist, double *rec, const int *rec_idx) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   {
     // the cell's own planes, before the annulus lookups they do not depend on
-    pf_planes(d.cons, 5, N, g);
+    pf_planes(d.cons, 5, QS, g);
     if (substep == 2) {
-      pf_planes(d.rkcons, 5, N, g);
+      pf_planes(d.rkcons, 5, QS, g);
       pf(d.rktiph + g);
     }
-    pf_planes(d.fphi, 8, N, g);
-    pf_planes(d.src, 6, N, g);
+    pf_planes(d.fphi, 8, QF, g);
+    pf_planes(d.src, 6, P8, g);
     pf(d.tiphw + g);
     pf((substep == 1 ? d.tiph0 : d.tiph1) + g);
     // and its r-face run ranges and first face, which k_merge just wrote
@@ -1286,10 +1327,9 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
     double cp[DGPU_MAX_PASSIVE], pp[DGPU_MAX_PASSIVE];
     const int np = PS ? P.num_n : 0;
     if (np > 0) passive_sum(d, A, a, g, substep, stop, np, cp);
-    if (!update_sum<T, !XC>(d, tp, A, a, g, substep, stop, dt, true, c)) {
-#pragma unroll
-      for (int q = 0; q < 5; ++q) stq<T>(d.cons, tp.cons, q, N, g, c[q]);
-      for (int k = 0; k < np; ++k) d.cons[(size_t)(5 + k) * N + g] = cp[k];
+    if (!update_sum<T, !XC, PS>(d, tp, A, a, g, substep, stop, dt, true, c)) {
+      stk<5, T>(d.cons, tp.cons, 0, QS, g, c);
+      for (int k = 0; k < np; ++k) d.cons[ix(5 + k, QS, g)] = cp[k];
     } else {
       double tn, rk;
       const double dphi_n = mesh_advance(d, A, a, g, substep, dt, tn, rk);
@@ -1297,10 +1337,12 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       (substep == 1 ? d.tiph1 : d.tiph0)[g] = tn;
       d.dphi[g] = dphi_n;
       if (rec) {
-        double *rs = rec + (size_t)(2 * (*rec_idx) + substep - 1) * 6 * N;
+        double *rs = rec + (size_t)(2 * (*rec_idx) + substep - 1) * 6 * d.n_pad;
+        double u[6];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) rs[(size_t)q * N + g] = val(c[q]);
-        rs[(size_t)5 * N + g] = dphi_n;
+        for (int q = 0; q < 5; ++q) u[q] = val(c[q]);
+        u[5] = dphi_n;
+        stk<6>(rs, 0, P6, g, u);
       }
       // cell_calc_prim -> cell_cons2prim (src/Cell/cell_conversion.c:57-122)
       const double r = .5 * (A.rm + A.rp);
@@ -1329,14 +1371,11 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
         prim2cons(pr, c, r, dV, P.gamma);
         for (int k = 0; k < np; ++k) cp[k] = pp[k] * val(c[D_DDD]);
       }
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        stq<T>(d.prim, tp.prim, q, N, g, pr[q]);
-        stq<T>(d.cons, tp.cons, q, N, g, c[q]);
-      }
+      stk<5, T>(d.prim, tp.prim, 0, QS, g, pr);
+      stk<5, T>(d.cons, tp.cons, 0, QS, g, c);
       for (int k = 0; k < np; ++k) {
-        d.prim[(size_t)(5 + k) * N + g] = pp[k];
-        d.cons[(size_t)(5 + k) * N + g] = cp[k];
+        d.prim[ix(5 + k, QS, g)] = pp[k];
+        d.cons[ix(5 + k, QS, g)] = cp[k];
       }
     }
   }
@@ -1676,19 +1715,17 @@ __global__ void __launch_bounds__(BLK, MB) k_sweep(const __grid_constant__ DevPt
 template <typename T, bool PS = false>
 __global__ void __launch_bounds__(BLK) k_calc_cons(DevPtrs d, TanPtrs tp) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = d.n_cells;
-  if (g >= N) return;
+  const Pl QS = {PS ? d.qs : 5};
+  if (g >= d.n_cells) return;
   const Annulus &A = d.ann[d.cell_ann[g]];
   const DiskParams &P = d.par[A.inst];
   double r = .5 * (A.rp + A.rm);
   double dV = A.dv_half * d.dphi[g] * A.dz;
   T p[5], c[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) p[q] = ldq<T>(d.prim, tp.prim, q, N, g);
+  ldk<5, T>(d.prim, tp.prim, 0, QS, g, p);
   prim2cons(p, c, r, dV, P.gamma);
-#pragma unroll
-  for (int q = 0; q < 5; ++q) stq<T>(d.cons, tp.cons, q, N, g, c[q]);
-  for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q) d.cons[(size_t)q * N + g] = ld(d.prim, q, N, g) * val(c[D_DDD]);
+  stk<5, T>(d.cons, tp.cons, 0, QS, g, c);
+  for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q) d.cons[ix(q, QS, g)] = ld(d.prim, q, QS, g) * val(c[D_DDD]);
 }
 
 // cell_boundary_outflow_r (src/Cell/cell_boundary.c:14-139) runs three passes
@@ -1770,7 +1807,8 @@ __global__ void __launch_bounds__(OUTFLOW_BLK) k_outflow(DevPtrs d, int stop) {
   const int lane = threadIdx.x & 31, sub = lane % OB_LANES, first = lane - sub;
   const unsigned group = ((1u << OB_LANES) - 1u) << first;
   if (t >= d.n_ob) return;
-  const int g = rd(d.ob_cell + t), N = d.n_cells;
+  const int g = rd(d.ob_cell + t);
+  const Pl QS = {PS ? d.qs : 5};
   const int a = rd(d.cell_ann + g);
   const Annulus &A = d.ann[a];
   if (!(A.kind & DGPU_AK_OUT_DST)) return;
@@ -1843,16 +1881,16 @@ __global__ void __launch_bounds__(OUTFLOW_BLK) k_outflow(DevPtrs d, int stop) {
   bc_damp(d, A, a, pr);
 #pragma unroll
   for (int q = 0; q < NQ; ++q)
-    if (!PS || q < nq) d.prim[(size_t)q * N + g] = pr[q];
+    if (!PS || q < nq) d.prim[ix(q, QS, g)] = pr[q];
   if (stop >= 7) {
     const double r = .5 * (A.rm + A.rp);
     const double dV = A.dv_half * dphi * A.dz;
     prim2cons(pr, c, r, dV, P.gamma);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) d.cons[(size_t)q * N + g] = c[q];
+    for (int q = 0; q < 5; ++q) d.cons[ix(q, QS, g)] = c[q];
 #pragma unroll
     for (int q = 5; q < NQ; ++q)
-      if (q < nq) d.cons[(size_t)q * N + g] = pr[q] * c[D_DDD];
+      if (q < nq) d.cons[ix(q, QS, g)] = pr[q] * c[D_DDD];
   }
 }
 
@@ -1864,7 +1902,6 @@ __global__ void __launch_bounds__(BLK) k_torque(DevPtrs d, int inst, double *par
   __shared__ bool last;
   const DiskParams &P = d.par[inst];
   const InstState &S = d.ist[inst];
-  const int N = d.n_cells;
   const int g = P.cell_base + blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0.0;
   if (g < P.cell_base + P.n_cells) {
@@ -1873,7 +1910,7 @@ __global__ void __launch_bounds__(BLK) k_torque(DevPtrs d, int inst, double *par
       double dphi = d.dphi[g];
       double phi = d.tiph0[g] - .5 * dphi;
       double r = .5 * (A.rp + A.rm);
-      double rho = ld(d.prim, D_RHO, N, g);
+      double rho = ld(d.prim, D_RHO, Pl{d.qs}, g);
       double dV = dphi * .5 * A.dv_diff * P.dz;
       double cosp = cos(phi), sinp = sin(phi);
       double Fp = 0.0;
@@ -1909,30 +1946,31 @@ __global__ void __launch_bounds__(BLK) k_torque(DevPtrs d, int inst, double *par
   d.counters[2] = 0;
 }
 
-// AoS rows [n][nq] (the boundary format) <-> SoA columns X[q*stride + base + c]
-__global__ void k_aos_to_soa(double *soa, int nq, int stride, int base, const double *aos, int n) {
+// AoS rows [n][nq] (the boundary format) <-> cells base .. base + n of an
+// array of `planes` planes
+__global__ void k_aos_to_soa(double *soa, int nq, Pl planes, int base, const double *aos, int n) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  for (int q = 0; q < nq; ++q) soa[(size_t)q * stride + base + c] = aos[(size_t)c * nq + q];
+  for (int q = 0; q < nq; ++q) soa[ix(q, planes, base + c)] = aos[(size_t)c * nq + q];
 }
-__global__ void k_soa_to_aos(double *aos, int nq, int stride, int base, const double *soa, int n) {
+__global__ void k_soa_to_aos(double *aos, int nq, Pl planes, int base, const double *soa, int n) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  for (int q = 0; q < nq; ++q) aos[(size_t)c * nq + q] = soa[(size_t)q * stride + base + c];
+  for (int q = 0; q < nq; ++q) aos[(size_t)c * nq + q] = soa[ix(q, planes, base + c)];
 }
 
 }  // namespace
 
 extern "C" {
 
-int dgk_aos_to_soa(double *soa, int nq, int stride, int base, const double *aos, int n, void *stream) {
+int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, void *stream) {
   if (n <= 0) return 0;
-  k_aos_to_soa<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(soa, nq, stride, base, aos, n);
+  k_aos_to_soa<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(soa, nq, Pl{planes}, base, aos, n);
   return (int)cudaGetLastError();
 }
-int dgk_soa_to_aos(double *aos, int nq, int stride, int base, const double *soa, int n, void *stream) {
+int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream) {
   if (n <= 0) return 0;
-  k_soa_to_aos<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(aos, nq, stride, base, soa, n);
+  k_soa_to_aos<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(aos, nq, Pl{planes}, base, soa, n);
   return (int)cudaGetLastError();
 }
 

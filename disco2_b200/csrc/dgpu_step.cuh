@@ -68,63 +68,63 @@ __device__ __forceinline__ double new_tiph(double tw, double &rk, double RK, dou
   return t;
 }
 
-// A face or source increment: through the read-only path (NC) when an earlier
-// kernel wrote it, by a plain load when another block of the running kernel
-// did.
-template <typename T, bool NC>
-__device__ __forceinline__ T ldinc(const double *v, const double *dv, int q, int n, int g) {
-  if constexpr (NC) return ldqr<T>(v, dv, q, n, g);
-  else return ldq<T>(v, dv, q, n, g);
-}
-
 // The conserved sum of a cell before cons2prim: cell_adjust_RK_cons, the phi
 // and r face increments in the reference's order, cell_add_src, cooling,
 // cell_add_visc_src and cell_add_split_fictitious (the forward stops after
 // `stop` like the stage-parity path; returns false when it stopped early).
 // Writes rkcons in substep 1 when `write_rk`.  NC: the increments and the
-// annulus constants come from earlier kernels (see ldinc).
-template <typename T, bool NC = true>
+// annulus constants come from earlier kernels (the read-only path), not from
+// another block of the running one (plain loads).
+template <typename T, bool NC = true, bool PS = false>
 __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, const Annulus &A, int a, int g,
                                            int substep, int stop, double dt, bool write_rk, T *c) {
-  const int N = d.n_cells;
+  const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   const DiskParams &P = d.par[A.inst];
   const int j = g - A.cell_off;
   const int np = A.np;
   const double RK = substep == 1 ? 0.0 : 0.5;
   // cell_copy (substep 1) + cell_adjust_RK_cons (cell_misc.c:28-57)
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    T cq = ldqr<T>(d.cons, tp.cons, q, N, g);
-    T rk;
+  {
+    T rk[5];
+    ldk<5, T, true>(d.cons, tp.cons, 0, QS, g, c);
     if (substep == 1) {
-      rk = cq;
-      if (write_rk) stq<T>(d.rkcons, tp.rkcons, q, N, g, cq);
+#pragma unroll
+      for (int q = 0; q < 5; ++q) rk[q] = c[q];
+      if (write_rk) stk<5, T>(d.rkcons, tp.rkcons, 0, QS, g, c);
     } else {
-      rk = ldqr<T>(d.rkcons, tp.rkcons, q, N, g);
+      ldk<5, T, true>(d.rkcons, tp.rkcons, 0, QS, g, rk);
     }
-    c[q] = (1.0 - RK) * cq + RK * rk;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) c[q] = (1.0 - RK) * c[q] + RK * rk[q];
   }
   if (stop <= 1) return false;
   // phi faces: for j = 0 the face (0,1) comes before (N-1,0)
   {
     const int gl = j == 0 ? A.cell_off + np - 1 : g - 1;
     const double r = .5 * (A.rp + A.rm);
+    // the eight increments of a face, the viscous ones after the others
     auto addL = [&](int f) {
+      T u[8];
+      if (P.has_visc) ldk<8, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
+      else ldk<5, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) c[q] -= ldinc<T, NC>(d.fphi, tp.fphi, q, N, f);
+      for (int q = 0; q < 5; ++q) c[q] -= u[q];
       if (P.has_visc) {
-        c[D_SRR] -= ldinc<T, NC>(d.fphi, tp.fphi, 5, N, f) / r;
-        c[D_LLL] -= ldinc<T, NC>(d.fphi, tp.fphi, 6, N, f);
-        c[D_TAU] -= ldinc<T, NC>(d.fphi, tp.fphi, 7, N, f);
+        c[D_SRR] -= u[5] / r;
+        c[D_LLL] -= u[6];
+        c[D_TAU] -= u[7];
       }
     };
     auto addR = [&](int f) {
+      T u[8];
+      if (P.has_visc) ldk<8, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
+      else ldk<5, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) c[q] += ldinc<T, NC>(d.fphi, tp.fphi, q, N, f);
+      for (int q = 0; q < 5; ++q) c[q] += u[q];
       if (P.has_visc) {
-        c[D_SRR] += ldinc<T, NC>(d.fphi, tp.fphi, 5, N, f) / r;
-        c[D_LLL] += ldinc<T, NC>(d.fphi, tp.fphi, 6, N, f);
-        c[D_TAU] += ldinc<T, NC>(d.fphi, tp.fphi, 7, N, f);
+        c[D_SRR] += u[5] / r;
+        c[D_LLL] += u[6];
+        c[D_TAU] += u[7];
       }
     };
     if (j == 0) {
@@ -139,7 +139,6 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   // r faces in face-list order, one face's increments at a time (two at a time
   // spill more at the kernel's 64-register budget)
   {
-    const int NS = d.n_slots;
     const bool visc = P.has_visc;
     for_cell_rface_ranges(d, A, a, g, P.NR, [&](int s, int e, int asR) {
       // the outer cell's faces divide the viscous S_r part by its own radius
@@ -166,9 +165,8 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
       };
       for (int n = s; n < e; ++n) {
         T u[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (q < 5 || visc) u[q] = ldinc<T, NC>(d.frf, tp.frf, q, NS, n);
+        if (visc) ldk<8, T, NC>(d.frf, tp.frf, 0, QF, n, u);
+        else ldk<5, T, NC>(d.frf, tp.frf, 0, QF, n, u);
         apply(u);
       }
     });
@@ -179,13 +177,11 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   // terms); adding its +0 to the upper cell keeps the reference's signed zeros.
   if constexpr (std::is_same<T, double>::value) {
     if (d.has_z && P.NZ > 1) {
-      const int NSZ = d.n_zslots;
       const bool visc = P.has_visc;
       for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int up) {
         for (int n = s; n < e; ++n) {
           double u[5];
-#pragma unroll
-          for (int q = 0; q < 5; ++q) u[q] = NC ? ldr(d.zfrf, q, NSZ, n) : ld(d.zfrf, q, NSZ, n);
+          ldk<5, NC>(d.zfrf, 0, P5, n, u);
           if (up) {
 #pragma unroll
             for (int q = 0; q < 5; ++q) c[q] += u[q];
@@ -205,19 +201,22 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   if (stop == 3) return false;
   // cell_add_src, cell_add_visc_src, cell_add_split_fictitious: the source
   // increments come from k_source; added here in the reference's order
-  c[D_SRR] += ldinc<T, NC>(d.src, tp.src, 0, N, g);
-  c[D_SRR] += ldinc<T, NC>(d.src, tp.src, 1, N, g);
-  c[D_LLL] += ldinc<T, NC>(d.src, tp.src, 2, N, g);
-  c[D_SZZ] += ldinc<T, NC>(d.src, tp.src, 3, N, g);
-  c[D_TAU] += ldinc<T, NC>(d.src, tp.src, 4, N, g);
+  T u[6];
+  ldk<6, T, NC>(d.src, tp.src, 0, P8, g, u);
+  c[D_SRR] += u[0];
+  c[D_SRR] += u[1];
+  c[D_LLL] += u[2];
+  c[D_SZZ] += u[3];
+  c[D_TAU] += u[4];
   if (P.rho_sink_on == 1) {
-    for (int p = 0; p < P.num_sinks && p < 2; ++p) c[D_DDD] -= ldinc<T, NC>(d.src, tp.src, 6 + p, N, g);
+    for (int p = 0; p < P.num_sinks && p < 2; ++p)
+      c[D_DDD] -= NC ? ldqr<T>(d.src, tp.src, 6 + p, P8, g) : ldq<T>(d.src, tp.src, 6 + p, P8, g);
   }
   const double rm = A.rm, rp = A.rp;
   const double r = .5 * (rp + rm);
   if (P.cooling == 1) {
     // cooling reads the running tau (cell_source.c:187-203)
-    const T rho = ldqr<T>(d.prim, tp.prim, D_RHO, N, g), Pp = ldqr<T>(d.prim, tp.prim, D_PPP, N, g);
+    const T rho = ldqr<T>(d.prim, tp.prim, D_RHO, QS, g), Pp = ldqr<T>(d.prim, tp.prim, D_PPP, QS, g);
     const double dV = rd(d.dphi + g) * .5 * A.dv_diff * A.dz;
     if (P.init_type == DI_SHEAR) {
       T cooling_term = (Pp - .01) / (P.gamma - 1.) * dV / 1.e-2;
@@ -232,7 +231,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
       c[D_TAU] -= cooling_term;
     }
   }
-  if (P.has_visc) c[D_TAU] += ldinc<T, NC>(d.src, tp.src, 5, N, g);
+  if (P.has_visc) c[D_TAU] += u[5];
   // cell_add_split_fictitious (src/Cell/cell_add_split_fictitious.c:11-44)
   {
     const double rom = frame_val(d, P, A.rom, a, DGPU_FR_ROM);
@@ -253,17 +252,17 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
 // substep 1.
 __device__ __forceinline__ void passive_sum(const DevPtrs &d, const Annulus &A, int a, int g, int substep,
                                             int stop, int np, double *cp) {
-  const int N = d.n_cells, NS = d.n_slots;
+  const Pl QS = {d.qs}, QF = {d.qf};
   const int j = g - A.cell_off;
   const double RK = substep == 1 ? 0.0 : 0.5;
   for (int k = 0; k < np; ++k) {
-    const double cq = ld(d.cons, 5 + k, N, g);
+    const double cq = ld(d.cons, 5 + k, QS, g);
     double rk;
     if (substep == 1) {
       rk = cq;
-      d.rkcons[(size_t)(5 + k) * N + g] = cq;
+      d.rkcons[ix(5 + k, QS, g)] = cq;
     } else {
-      rk = ld(d.rkcons, 5 + k, N, g);
+      rk = ld(d.rkcons, 5 + k, QS, g);
     }
     cp[k] = (1.0 - RK) * cq + RK * rk;
   }
@@ -272,11 +271,11 @@ __device__ __forceinline__ void passive_sum(const DevPtrs &d, const Annulus &A, 
     const int gl = j == 0 ? A.cell_off + A.np - 1 : g - 1;
     for (int k = 0; k < np; ++k) {
       if (j == 0) {
-        cp[k] -= ld(d.fphi, 8 + k, N, g);
-        cp[k] += ld(d.fphi, 8 + k, N, gl);
+        cp[k] -= ld(d.fphi, 8 + k, QF, g);
+        cp[k] += ld(d.fphi, 8 + k, QF, gl);
       } else {
-        cp[k] += ld(d.fphi, 8 + k, N, gl);
-        cp[k] -= ld(d.fphi, 8 + k, N, g);
+        cp[k] += ld(d.fphi, 8 + k, QF, gl);
+        cp[k] -= ld(d.fphi, 8 + k, QF, g);
       }
     }
   }
@@ -284,8 +283,8 @@ __device__ __forceinline__ void passive_sum(const DevPtrs &d, const Annulus &A, 
   for_cell_rface_ranges(d, A, a, g, d.par[A.inst].NR, [&](int s, int e, int asR) {
     for (int n = s; n < e; ++n)
       for (int k = 0; k < np; ++k) {
-        if (asR) cp[k] += ld(d.frf, 8 + k, NS, n);
-        else cp[k] -= ld(d.frf, 8 + k, NS, n);
+        if (asR) cp[k] += ld(d.frf, 8 + k, QF, n);
+        else cp[k] -= ld(d.frf, 8 + k, QF, n);
       }
   });
 }
