@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_ADJ) a_update_source(DevPtrs d,
       const double dV = A.dv_half * dphi_n * P.dz;
       double pr[5];
       cons2prim(c, dV, r, P, pr);
-      bc_damp<double>(d, A, a, pr);
+      bc_damp(d, A, a, pr);
       double apr[5], alc[5];
 #pragma unroll
       for (int q = 0; q < 5; ++q) {

@@ -218,7 +218,7 @@ void dgpu_destroy(dgpu_ctx *c) {
                   c->d.rkcons, c->d.grad, c->d.gradp, c->d.tiph0, c->d.tiph1, c->d.tiphw, c->d.rktiph,
                   c->d.dphi, c->d.w_ann, c->d.frame, c->d.fphi, c->d.frf, c->d.fS, c->d.fdp, c->d.ann_c, c->d.src, c->d.rr, c->d.fstart, c->d.fL, c->d.fR, c->d.fdphi,
                   c->d.fcm, c->d.pair_nf, c->d.pair_jpmin, c->d.pair_T, c->d.pair_seq, c->d.runs,
-                  c->d.mdot_part, c->d.counters, c->d.err, c->d.obuf, c->d_ob_cell, c->d_stage, c->d_torque,
+                  c->d.mdot_part, c->d.counters, c->d.err, c->d.obuf, c->d_ob_cell, c->d_vz, c->d_stage, c->d_torque,
                   c->d.cfl_ann, c->d.sweep_flag, c->d_zslot_ann, c->d.zfL, c->d.zfR, c->d.zfdphi, c->d.zfcm,
                   c->d.zfstart, c->d.zrr, c->d.zruns, c->d.zpair_nf, c->d.zpair_jpmin, c->d.zpair_T,
                   c->d.zpair_seq, c->d.zfS, c->d.zfdp, c->d.zfrf, c->d.gradz};
@@ -236,6 +236,7 @@ void dgpu_destroy(dgpu_ctx *c) {
   }
   free(c->h_par);
   free(c->h_ann);
+  free(c->vz_always);
   free(c);
 }
 
@@ -445,6 +446,9 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
       c->d.gradz = (double *)dmalloc(sizeof(double) * 5 * N, &ok);
     }
     c->d.err = (int *)dmalloc(sizeof(int), &ok);
+    c->d_vz = (int *)dmalloc(sizeof(int) * (1 + (size_t)n), &ok);
+    c->vz_always = (int *)calloc((size_t)n, sizeof(int));
+    if (!c->vz_always) ok = 0;
     if (n_ob > 0) {
       c->d.obuf = (double *)dmalloc(sizeof(double) * NQ * (size_t)n_ob, &ok);
       c->d_ob_cell = (int *)dmalloc(sizeof(int) * (size_t)n_ob, &ok);
@@ -507,6 +511,17 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   c->d.cell_ann = c->d_cell_ann;
   c->d.slot_ann = c->d_slot_ann;
   c->d.ob_cell = c->d_ob_cell;
+  /* v_z stays 0 where it starts so if no layer's gravity has a vertical part
+   * (2-D; Grav_2D, or the layer at z = 0) and no boundary target has a v_z;
+   * until its first upload every disk counts as having one */
+  c->d.vz = c->d_vz;
+  for (k = 0; k < n; ++k) {
+    const DiskParams *p = &c->h_par[k];
+    c->vz_always[k] = p->NZ > 1 || !(p->grav2d == 1 || p->z == 0.0);
+  }
+  for (i = 0; i < c->n_ann; ++i)
+    if (c->h_ann[i].ic[D_UZZ] != 0.0) c->vz_always[c->h_ann[i].inst] = 1;
+  cudaMemset(c->d_vz, 1, sizeof(int) * (1 + (size_t)n));
   c->d.ob_three = 0;
   for (k = 0; k < n; ++k)
     if ((c->h_par[k].outflow & 1) && c->h_par[k].NR == 3) c->d.ob_three = 1;
@@ -592,7 +607,9 @@ static int upload_disk(struct dgpu_ctx *c, int inst, const double *prim, const d
   if (prim) {
     const int nq = 5 + p->num_n;
     CK(cudaMemcpyAsync(c->d_stage, prim, sizeof(double) * nq * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    CKK(dgk_aos_to_soa(c->d.prim, nq, c->d.qs, base, c->d_stage, n, c->stream));
+    CK(cudaMemsetAsync(c->d_vz + 1 + inst, c->vz_always[inst], sizeof(int), c->stream));
+    CKK(dgk_aos_to_soa(c->d.prim, nq, c->d.qs, base, c->d_stage, n, c->d_vz + 1 + inst, c->stream));
+    CKK(dgk_any_vz(c->d_vz, c->n_inst, c->stream));
   }
   if (tiph) CK(cudaMemcpyAsync(c->d.tiph0 + base, tiph, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
   if (dphi) CK(cudaMemcpyAsync(c->d.dphi + base, dphi, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
@@ -1060,26 +1077,32 @@ int dgpu_stage(dgpu_ctx *c, int phase) {
   if (!c || phase < 0 || phase > 15) return DGPU_ERR_ARG;
   if (c->d.has_z) return fail(c, DGPU_ERR_UNSUPPORTED, "stage parity of 3-D disks (NumZ > 1) is not implemented");
   cudaSetDevice(c->device);
+  DevPtrs h = c->d; /* with every plane, which dgpu_get_stage_data returns */
+  h.vz = NULL;
   /* phases 8-15: the whole first substep (its k_update also moves the
    * GravMass, as timestep_rk2 does between the substeps), then the second */
   if (sub == 2) {
-    int rc = dctx_substep(c, NULL, 1);
+    const int *vz = c->d.vz;
+    int rc;
+    c->d.vz = NULL;
+    rc = dctx_substep(c, NULL, 1);
+    c->d.vz = vz;
     if (rc) return rc;
   }
-  CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
-  CKK(dgk_merge(&c->d, sub, c->stream));
+  CKK(dgk_cellprep(&h, NULL, sub, c->stream));
+  CKK(dgk_merge(&h, sub, c->stream));
   /* the CFL minimum comes from k_plm_r (and dt from it, stored here for the
    * phases before k_update stores it); PLM results are kept only from phase 1 on */
-  CKK(dgk_rslope(&c->d, NULL, c->stream));
-  CKK(dgk_plm_r(&c->d, NULL, sub, c->stream));
-  if (sub == 1) CKK(dgk_dt(&c->d, c->stream));
-  CKK(dgk_source(&c->d, NULL, sub, c->stream));
+  CKK(dgk_rslope(&h, NULL, c->stream));
+  CKK(dgk_plm_r(&h, NULL, sub, c->stream));
+  if (sub == 1) CKK(dgk_dt(&h, c->stream));
+  CKK(dgk_source(&h, NULL, sub, c->stream));
   if (stop >= 2) {
-    CKK(dgk_flux_phi(&c->d, NULL, sub, c->stream));
-    CKK(dgk_flux_r(&c->d, NULL, sub, c->stream));
+    CKK(dgk_flux_phi(&h, NULL, sub, c->stream));
+    CKK(dgk_flux_r(&h, NULL, sub, c->stream));
   }
-  CKK(dgk_update_stage(&c->d, sub, stop, c->stream));
-  if (stop >= 6 && c->n_ob > 0) CKK(dgk_outflow(&c->d, stop, c->stream));
+  CKK(dgk_update_stage(&h, sub, stop, c->stream));
+  if (stop >= 6 && c->n_ob > 0) CKK(dgk_outflow(&h, stop, c->stream));
   /* from phase 5 of substep 1 on the advanced phi edges live in the substep's
    * output buffer (substep 2 writes them where the state is read) */
   if (sub == 1 && stop >= 5)

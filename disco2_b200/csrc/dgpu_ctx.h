@@ -32,6 +32,8 @@ struct dgpu_ctx {
   InstState *d_ist;
   Annulus *d_ann;
   int *d_cell_ann, *d_slot_ann, *d_zslot_ann, *d_ob_cell;
+  int *d_vz;          /* [1 + n_inst] v_z flags: any disk's, then each disk's (upload_disk) */
+  int *vz_always;     /* [n_inst] disks whose v_z cannot be left out whatever their prims */
   double *d_stage;    /* AoS staging buffer: max cells of a disk x NQ */
   double *d_torque;   /* partial sums + result */
   cudaGraphExec_t graph;

@@ -359,40 +359,48 @@ HD T fgrav(const T &M, const T &r, double eps, int n) {
 // _set_star_hllc and the flux choice of riemann_AddFlux
 // (src/Riemann/Riemann_routines.c:14-191,314-371).  dir 0 = r face, 1 = phi, 2 = z.
 // ---------------------------------------------------------------------------
-template <typename T>
+//
+// NV = 4: the disk has no v_z (see no_vz).  The terms left out are exact
+// zeros, so the others keep their values; plane UZZ / SZZ is neither read nor
+// written.
+template <int NV = 5, typename T>
 HD void phys_flux(const T *p, double r, double n0, double n1, double n2, double gam, T *F) {
   T rho = p[D_RHO];
   T Pp = p[D_PPP];
   T vr = p[D_URR];
   T vp = p[D_UPP] * r;
-  T vz = p[D_UZZ];
-  T vn = vr * n0 + vp * n1 + vz * n2;
+  T vn = vr * n0 + vp * n1;
   T rhoe = Pp / (gam - 1.);
-  T v2 = vr * vr + vp * vp + vz * vz;
+  T v2 = vr * vr + vp * vp;
+  if constexpr (NV == 5) {
+    T vz = p[D_UZZ];
+    vn = vn + vz * n2;
+    v2 = v2 + vz * vz;
+  }
   F[D_DDD] = rho * vn;
   F[D_SRR] = rho * vr * vn + Pp * n0;
   F[D_LLL] = r * (rho * vp * vn + Pp * n1);
-  F[D_SZZ] = rho * vz * vn + Pp * n2;
+  if constexpr (NV == 5) F[D_SZZ] = rho * p[D_UZZ] * vn + Pp * n2;
   F[D_TAU] = (.5 * rho * v2 + rhoe + Pp) * vn;
 }
 // cell_prim2cons (src/Cell/cell_conversion.c:11-33)
-template <typename T>
+template <int NV = 5, typename T>
 HD void prim2cons(const T *p, T *U, double r, double dV, double gam) {
   T rho = p[D_RHO];
   T Pp = p[D_PPP];
   T vr = p[D_URR];
   T vp = p[D_UPP] * r;
-  T vz = p[D_UZZ];
-  T v2 = vr * vr + vp * vp + vz * vz;
+  T v2 = vr * vr + vp * vp;
+  if constexpr (NV == 5) v2 = v2 + p[D_UZZ] * p[D_UZZ];
   T rhoe = Pp / (gam - 1.);
   U[D_DDD] = rho * dV;
   U[D_SRR] = rho * vr * dV;
   U[D_LLL] = r * rho * vp * dV;
-  U[D_SZZ] = rho * vz * dV;
+  if constexpr (NV == 5) U[D_SZZ] = rho * p[D_UZZ] * dV;
   U[D_TAU] = (.5 * rho * v2 + rhoe) * dV;
 }
 
-template <typename T>
+template <int NV = 5, typename T>
 // np passive scalars (face states qL, qR) ride on the mass flux: their
 // physical flux and conserved value are q F_D and q U_D (riemann_set_flux,
 // Riemann_routines.c:184-189; cell_prim2cons, cell_conversion.c:28-31), their
@@ -404,13 +412,15 @@ HD void riemann_flux(const T *pL, const T *pR, double r, int dir, double w, doub
   const double n0 = dir == 0 ? 1.0 : 0.0, n1 = dir == 1 ? 1.0 : 0.0, n2 = dir == 2 ? 1.0 : 0.0;
   T vnL, cf2L, vnR, cf2R;
   {
-    T P = pL[D_PPP], rho = pL[D_RHO], vr = pL[D_URR], vp = r * pL[D_UPP], vz = pL[D_UZZ];
-    vnL = vr * n0 + vp * n1 + vz * n2;
+    T P = pL[D_PPP], rho = pL[D_RHO], vr = pL[D_URR], vp = r * pL[D_UPP];
+    vnL = vr * n0 + vp * n1;
+    if constexpr (NV == 5) vnL = vnL + pL[D_UZZ] * n2;
     cf2L = gam * (P / rho);
   }
   {
-    T P = pR[D_PPP], rho = pR[D_RHO], vr = pR[D_URR], vp = r * pR[D_UPP], vz = pR[D_UZZ];
-    vnR = vr * n0 + vp * n1 + vz * n2;
+    T P = pR[D_PPP], rho = pR[D_RHO], vr = pR[D_URR], vp = r * pR[D_UPP];
+    vnR = vr * n0 + vp * n1;
+    if constexpr (NV == 5) vnR = vnR + pR[D_UZZ] * n2;
     cf2R = gam * (P / rho);
   }
   T Sl = vnL - sqrt(cf2L);
@@ -428,10 +438,10 @@ HD void riemann_flux(const T *pL, const T *pR, double r, int dir, double w, doub
   T Fk[5], Uk[5];
   if (state == DS_LEFT || state == DS_RIGHT) {
     const T *p = state == DS_LEFT ? pL : pR;
-    phys_flux(p, r, n0, n1, n2, gam, Fk);
-    prim2cons(p, Uk, r, 1.0, gam);
+    phys_flux<NV>(p, r, n0, n1, n2, gam, Fk);
+    prim2cons<NV>(p, Uk, r, 1.0, gam);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) F[q] = Fk[q] - w * Uk[q];
+    for (int q = 0; q < NV; ++q) F[q] = Fk[q] - w * Uk[q];
     for (int k = 0; k < np; ++k) {
       const double qk = state == DS_LEFT ? qL[k] : qR[k];
       const double Fkq = qk * val(Fk[D_DDD]), Ukq = qk * val(Uk[D_DDD]);
@@ -442,12 +452,12 @@ HD void riemann_flux(const T *pL, const T *pR, double r, int dir, double w, doub
   T Ustar[5], Fstar[5];
   if (solver == DR_HLL) {
     T FL[5], FR[5], UL[5], UR[5];
-    phys_flux(pL, r, n0, n1, n2, gam, FL);
-    phys_flux(pR, r, n0, n1, n2, gam, FR);
-    prim2cons(pL, UL, r, 1.0, gam);
-    prim2cons(pR, UR, r, 1.0, gam);
+    phys_flux<NV>(pL, r, n0, n1, n2, gam, FL);
+    phys_flux<NV>(pR, r, n0, n1, n2, gam, FR);
+    prim2cons<NV>(pL, UL, r, 1.0, gam);
+    prim2cons<NV>(pR, UR, r, 1.0, gam);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
+    for (int q = 0; q < NV; ++q) {
       Ustar[q] = (Sr * UR[q] - Sl * UL[q] + FL[q] - FR[q]) / (Sr - Sl);
       Fstar[q] = (Sr * FL[q] - Sl * FR[q] - Sr * Sl * (UL[q] - UR[q])) / (Sr - Sl);
     }
@@ -462,39 +472,44 @@ HD void riemann_flux(const T *pL, const T *pR, double r, int dir, double w, doub
   } else {
     const T *prim = state == DS_LEFTSTAR ? pL : pR;
     T Sk = state == DS_LEFTSTAR ? Sl : Sr;
-    phys_flux(prim, r, n0, n1, n2, gam, Fk);
-    prim2cons(prim, Uk, r, 1.0, gam);
+    phys_flux<NV>(prim, r, n0, n1, n2, gam, Fk);
+    prim2cons<NV>(prim, Uk, r, 1.0, gam);
     T rho = prim[D_RHO];
     T vr = prim[D_URR];
     T vp = prim[D_UPP] * r;
-    T vz = prim[D_UZZ];
     T Pp = prim[D_PPP];
-    T v2 = vr * vr + vp * vp + vz * vz;
-    T vn = vr * n0 + vp * n1 + vz * n2;
+    T v2 = vr * vr + vp * vp;
+    T vn = vr * n0 + vp * n1;
+    if constexpr (NV == 5) {
+      T vz = prim[D_UZZ];
+      v2 = v2 + vz * vz;
+      vn = vn + vz * n2;
+    }
     T rhoe = Pp / (gam - 1.);
     T D = rho;
     T mr = rho * vr;
     T mp = rho * vp;
-    T mz = rho * vz;
     T E_hydro = .5 * rho * v2 + rhoe;
     T Ps = rho * (Sk - vn) * (Ss - vn) + Pp;
     T Dstar = (Sk - vn) * D / (Sk - Ss);
     T Msn = Dstar * Ss;
     T Msr = (Sk - vn) * mr / (Sk - Ss);
     T Msp = (Sk - vn) * mp / (Sk - Ss);
-    T Msz = (Sk - vn) * mz / (Sk - Ss);
+    T Msz = 0.0;
+    if constexpr (NV == 5) Msz = (Sk - vn) * (rho * prim[D_UZZ]) / (Sk - Ss);
     T Estar = ((Sk - vn) * E_hydro + Ps * Ss - Pp * vn) / (Sk - Ss);
-    T mn = Msr * n0 + Msp * n1 + Msz * n2;
+    T mn = Msr * n0 + Msp * n1;
+    if constexpr (NV == 5) mn = mn + Msz * n2;
     Msr += n0 * (Msn - mn);
     Msp += n1 * (Msn - mn);
-    Msz += n2 * (Msn - mn);
+    if constexpr (NV == 5) Msz += n2 * (Msn - mn);
     Ustar[D_DDD] = Dstar;
     Ustar[D_SRR] = Msr;
     Ustar[D_LLL] = r * Msp;
-    Ustar[D_SZZ] = Msz;
+    if constexpr (NV == 5) Ustar[D_SZZ] = Msz;
     Ustar[D_TAU] = Estar;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) Fstar[q] = Fk[q] + Sk * (Ustar[q] - Uk[q]);
+    for (int q = 0; q < NV; ++q) Fstar[q] = Fk[q] + Sk * (Ustar[q] - Uk[q]);
     for (int k = 0; k < np; ++k) {
       const double qk = state == DS_LEFTSTAR ? qL[k] : qR[k];
       const double Fkq = qk * val(Fk[D_DDD]), Ukq = qk * val(Uk[D_DDD]);
@@ -504,7 +519,7 @@ HD void riemann_flux(const T *pL, const T *pR, double r, int dir, double w, doub
     }
   }
 #pragma unroll
-  for (int q = 0; q < 5; ++q) F[q] = Fstar[q] - w * Ustar[q];
+  for (int q = 0; q < NV; ++q) F[q] = Fstar[q] - w * Ustar[q];
 }
 
 // Inputs of riemann_visc_flux (src/Riemann/Riemann_routines.c:193-311).
@@ -529,7 +544,7 @@ struct GravT {
 // from the reconstructed states first and then overwrites them (r faces: Avg
 // and Gr from the cell prims offset to the face centre; phi faces: Avg and Gp
 // from the cell prims), so the reconstructed states never reach the flux.
-template <typename T>
+template <int NV = 5, typename T>
 HD void visc_flux(const ViscIn<T> &v, int dir, const DiskParams &P, const GravT<T> &G, T *Fv, int *err) {
   const double r = v.r;
   T Avg[5], Gr[5], Gp[5];
@@ -553,7 +568,7 @@ HD void visc_flux(const ViscIn<T> &v, int dir, const DiskParams &P, const GravT<
       Gr[q] = .5 * (v.grL[q] + v.grR[q]);
     }
   }
-  {
+  if constexpr (NV == 5) {
     // the v_z check of the reference (Riemann_routines.c:271-274)
     double vz = dir == 0 ? .5 * ((val(v.cL[D_UZZ]) + v.dpL * val(v.gpL[D_UZZ])) +
                                  (val(v.cR[D_UZZ]) - v.dpR * val(v.gpR[D_UZZ])))
@@ -621,13 +636,12 @@ struct SrcGeom {
 // Source increments s[0..5] (S_r pressure/centrifugal, S_r gravity + frame, L,
 // S_z, tau, viscous heating) from the prims, grad[UPP], gradp[URR] and the
 // binary; sinks are handled by the caller.
-template <typename T>
+template <int NV = 5, typename T>
 HD void source_cell(const SrcGeom &g, const DiskParams &P, const T *pm, const T &grad_upp, const T &gradp_urr,
                     const GravT<T> &G, T *s) {
   T rho = pm[D_RHO];
   T Pp = pm[D_PPP];
   T vr = pm[D_URR];
-  T vz = pm[D_UZZ];
   T vp = pm[D_UPP] * g.r;
   T Fr = 0.0, Fp = 0.0;
   for (int p = 0; p < 2; ++p) {
@@ -647,8 +661,12 @@ HD void source_cell(const SrcGeom &g, const DiskParams &P, const T *pm, const T 
   s[0] = g.dt * g.dV * (rho * vp * vp + Pp) / g.r;
   s[1] = g.dt * g.dV * rho * (Fr * g.sint + g.Fc);
   s[2] = g.dt * g.dV * rho * (Fp - g.r * g.dtOm) * g.r;
-  s[3] = g.dt * g.dV * rho * Fr * g.cost;
-  s[4] = g.dt * g.dV * rho * ((Fr * g.sint + g.Fc) * vr + Fr * vz * g.cost + (Fp + F_euler_phi) * vp);
+  T work = (Fr * g.sint + g.Fc) * vr;
+  if constexpr (NV == 5) {
+    s[3] = g.dt * g.dV * rho * Fr * g.cost;
+    work = work + Fr * pm[D_UZZ] * g.cost;
+  }
+  s[4] = g.dt * g.dV * rho * (work + (Fp + F_euler_phi) * vp);
   s[5] = 0.0;
   if (P.has_visc) {
     T dist_bh0 = sqrt((g.xpos - G.gx[0]) * (g.xpos - G.gx[0]) + (g.ypos - G.gy[0]) * (g.ypos - G.gy[0]));
@@ -680,18 +698,22 @@ HD void split_rotate(T *c, double ck, double sk, double dr_r2Om, double kappa, d
 
 // cell_cons2prim (src/Cell/cell_conversion.c:57-122): density floor, sound-
 // speed floor and cap, velocity cap.
-template <typename T>
+template <int NV = 5, typename T>
 HD void cons2prim(const T *c, double dV, double r, const DiskParams &P, T *pr) {
   T rho = c[D_DDD] / dV;
   if (rho < P.rho_floor) rho = P.rho_floor;
   T Sr = c[D_SRR] / dV;
   T Sp = c[D_LLL] / dV / r;
-  T Sz = c[D_SZZ] / dV;
   T E = c[D_TAU] / dV;
   T vr = Sr / rho;
   T vp = Sp / rho;
-  T vz = Sz / rho;
-  T KE = .5 * (Sr * vr + Sp * vp + Sz * vz);
+  T S2 = Sr * vr + Sp * vp, vz = 0.0;
+  if constexpr (NV == 5) {
+    T Sz = c[D_SZZ] / dV;
+    vz = Sz / rho;
+    S2 = S2 + Sz * vz;
+  }
+  T KE = .5 * S2;
   T v_magnitude = sqrt(2. * KE / rho);
   T rhoe = E - KE;
   T Pp = (P.gamma - 1.) * rhoe;
@@ -700,13 +722,13 @@ HD void cons2prim(const T *c, double dV, double r, const DiskParams &P, T *pr) {
   if (v_magnitude > P.vel_cap) {
     vr = vr * P.vel_cap / v_magnitude;
     vp = vp * P.vel_cap / v_magnitude;
-    vz = vz * P.vel_cap / v_magnitude;
+    if constexpr (NV == 5) vz = vz * P.vel_cap / v_magnitude;
   }
   pr[D_RHO] = rho;
   pr[D_PPP] = Pp;
   pr[D_URR] = vr;
   pr[D_UPP] = vp / r;
-  pr[D_UZZ] = vz;
+  if constexpr (NV == 5) pr[D_UZZ] = vz;
 }
 
 // ---------------------------------------------------------------------------

@@ -338,6 +338,7 @@ static int alloc_shadow(struct dgpu_ctx *c, DevPtrs *h, void **mem) {
   CK(cudaMemset(*mem, 0, off[k]));
   m = (char *)*mem;
   *h = c->d;
+  h->vz = NULL; /* the reverse kernels read every plane */
   h->prim = (double *)(m + off[0]);
   h->cons = h->prim + 5 * N;
   h->rkcons = h->cons + 5 * N;
@@ -625,7 +626,7 @@ int dgpu_tangent(dgpu_ctx *c, int nsteps, int window_start, double dq_dir, doubl
   if (dprim) {
     CK(cudaMemcpyAsync(c->d_stage, dprim, sizeof(double) * 5 * (size_t)c->n_cells, cudaMemcpyHostToDevice,
                        c->stream));
-    CKK(dgk_aos_to_soa(D->t.prim, 5, c->d.qs, 0, c->d_stage, c->n_cells, c->stream));
+    CKK(dgk_aos_to_soa(D->t.prim, 5, c->d.qs, 0, c->d_stage, c->n_cells, NULL, c->stream));
   }
   CKK(dgk_calc_cons(&c->d, &D->t, c->stream));
   CKK(dgk_set_int(D->d_idx, 0, c->stream));

@@ -169,6 +169,7 @@ typedef struct {
   double *fS;             /* [5][n_slots] r-face slopes (WR - WL)/(deltaR + deltaL) */
   double *fdp;            /* [2][n_slots] r-face offsets dpL, dpR (wrapped to [-pi, pi]) */
   double *ann_c;          /* [4][n_ann] per substep: kappa, cos(kappa dt), sin(kappa dt), 1-exp(-rate dt) */
+  const int *vz;          /* vz[0]: some disk may have a v_z (no_vz); NULL: taken as so */
   int form_dt;            /* substep 1 forms dt from dtkey where it is read (step_dt); 0: dgk_dt or
                              dgk_set_dt has stored it */
   int smem_face;          /* dynamic shared bytes of k_merge (0: merge reads global memory) */
@@ -317,7 +318,8 @@ int dgk_diagnostics(const DevPtrs *d, int inst, int n_ann_disk, double *rows, do
 int dgk_torque(const DevPtrs *d, int inst, double *part, double *out, int n_inst_cells, void *stream);
 int dgk_update_blocks(int n_cells);
 int dgk_block_size(void);
-int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, void *stream);
+int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, int *vz, void *stream);
+int dgk_any_vz(int *vz, int n_inst, void *stream);
 int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream);
 #ifdef __cplusplus
 }

@@ -180,11 +180,11 @@ __device__ T block_excl_scan(T v, T *sh, T &total) {
 
 // Per cell, once per substep: cell_clean_pi of the phi edge
 // (src/Cell/cell_misc.c:12-26) and cell_plm_p (src/Cell/cell_plm.c:116-161).
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void cellprep_cell(const DevPtrs &d, const TanPtrs &tp, int g, int substep) {
   const Pl QS = {PS ? d.qs : 5};
   const double *traw = substep == 1 ? d.tiph0 : d.tiph1;
-  pf_planes(d.prim, 5, QS, g);
+  pf_planes(d.prim, NV, QS, g);
   pf(d.dphi + g);
   pf(traw + g);
   const int a = d.cell_ann[g];
@@ -210,20 +210,29 @@ __device__ __forceinline__ void cellprep_cell(const DevPtrs &d, const TanPtrs &t
   };
   slopes(std::integral_constant<int, 2>(), 0);
   slopes(std::integral_constant<int, 2>(), 2);
-  slopes(std::integral_constant<int, 1>(), 4);
+  if constexpr (NV == 5) slopes(std::integral_constant<int, 1>(), 4);
   for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q)
     d.gradp[ix(q, QS, g)] =
         plm_p_slope(ld(d.prim, q, QS, gl), ld(d.prim, q, QS, g), ld(d.prim, q, QS, gr), dpL, dpR, P.plm);
 }
 
+// Instances that carry the four-plane form (no_vz) beside the five: the plain
+// forward ones.  Each also exists without it (V4 = false), for contexts that
+// can never take it (3-D disks) and for the reverse sweep's replays: the two
+// forms in one kernel share its register budget, which cost the 3-D torus 5%
+// of its step.
+template <typename T, bool PS>
+constexpr bool forward_v4 = std::is_same<T, double>::value && !PS;
+
 // cellprep_cell for every cell and, for the first cell of each disk,
 // gravMass_copy at the start of a step (GravMass_misc.c:20-28) and
 // gravMass_clean_pi (GravMass_misc.c:9-17).  Runs concurrently with k_merge.
-template <typename T, bool PS = false>
+template <typename T, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(BLK, DGPU_MINB_CELLPREP) k_cellprep(DevPtrs d, TanPtrs tp, int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.n_cells) return;
-  cellprep_cell<T, PS>(d, tp, g, substep);
+  if (V4 && no_vz(d)) cellprep_cell<T, PS, V4 ? 4 : 5>(d, tp, g, substep);
+  else cellprep_cell<T, PS>(d, tp, g, substep);
   const Annulus &A = d.ann[d.cell_ann[g]];
   const DiskParams &P = d.par[A.inst];
   if (g == P.cell_base) {
@@ -542,16 +551,16 @@ __global__ void __launch_bounds__(BLK, DGPU_MINB_FACE) k_zmerge(DevPtrs d, int s
 // cell_plm_rz (src/Cell/cell_plm.c:31-53) and the wrapped dpL, dpR that
 // cell_plm_rz, riemann_setup_rz (Riemann_setup.c:18-25) and riemann_visc_flux
 // (Riemann_routines.c:220-228) all form the same way.
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void rslope_face(const DevPtrs &d, const TanPtrs &tp, int slot) {
   const int cL = rd(d.fL + slot);
   if (cL < 0) return;  // slot past the face list of its pair
   const int cR = rd(d.fR + slot);
   const Pl QS = {PS ? d.qs : 5};
-  pf_planes(d.prim, 5, QS, cL);
-  pf_planes(d.prim, 5, QS, cR);
-  pf_planes(d.gradp, 5, QS, cL);
-  pf_planes(d.gradp, 5, QS, cR);
+  pf_planes(d.prim, NV, QS, cL);
+  pf_planes(d.prim, NV, QS, cR);
+  pf_planes(d.gradp, NV, QS, cL);
+  pf_planes(d.gradp, NV, QS, cR);
   const int a = rd(d.slot_ann + slot);
   const Annulus &A = d.ann[a];
   const double cm = rd(d.fcm + slot);
@@ -565,7 +574,7 @@ __device__ __forceinline__ void rslope_face(const DevPtrs &d, const TanPtrs &tp,
   stk<2>(d.fdp, 0, P2, slot, dp);
   const double den = A.f_dr + A.f_dl;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
+  for (int q = 0; q < NV; ++q) {
     const T WL = ldqr<T>(d.prim, tp.prim, q, QS, cL) + dpL * ldqr<T>(d.gradp, tp.gradp, q, QS, cL);
     const T WR = ldqr<T>(d.prim, tp.prim, q, QS, cR) - dpR * ldqr<T>(d.gradp, tp.gradp, q, QS, cR);
     stq<T>(d.fS, tp.fS, q, QS, slot, (WR - WL) / den);
@@ -577,11 +586,12 @@ __device__ __forceinline__ void rslope_face(const DevPtrs &d, const TanPtrs &tp,
   }
 }
 
-template <typename T, bool PS = false>
+template <typename T, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(BLK) k_rslope(DevPtrs d, TanPtrs tp) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= d.n_slots) return;
-  rslope_face<T, PS>(d, tp, slot);
+  if (V4 && no_vz(d)) rslope_face<T, PS, V4 ? 4 : 5>(d, tp, slot);
+  else rslope_face<T, PS>(d, tp, slot);
 }
 
 // cell_plm_rz's limiter of plane q (src/Cell/cell_plm.c:81-113) as the
@@ -617,7 +627,7 @@ __device__ __noinline__ void limit_seq(const DevPtrs &d, const TanPtrs &tp, int 
 // here from the cell across the face, with no slopes stored, took 495 us for
 // the 191 and k_rslope's 200: the walk is as long as the longest lane's, and a
 // face-parallel kernel has no such waste.
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, int g) {
   const Pl QS = {PS ? d.qs : 5};
   pf(d.rr + 4 * (size_t)g);
@@ -630,7 +640,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
   T gq[5], lim[5];
   int neg = 0, pos = 0;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
+  for (int q = 0; q < NV; ++q) {
     gq[q] = 0.0;
     lim[q] = HUGE_VAL;
   }
@@ -640,9 +650,9 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
     for (int n = s; n < e; ++n) {
       const double dA = fr * rd(d.fdphi + n) * fperp;
       T Sf[5];
-      ldk<5, T>(d.fS, tp.fS, 0, QS, n, Sf);
+      ldk<NV, T>(d.fS, tp.fS, 0, QS, n, Sf);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
+      for (int q = 0; q < NV; ++q) {
         const T S = Sf[q];
         gq[q] += S * dA;
         const T ps = plm * S;
@@ -661,7 +671,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
   }
   int seq = 0;  // planes that run the loop itself
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
+  for (int q = 0; q < NV; ++q) {
     T m = gq[q] / dAtot;
     if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
       // every product S * m is at least |lim| |m| / plm in size
@@ -672,7 +682,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
     }
     gq[q] = m;
   }
-  stk<5, T>(d.grad, tp.grad, 0, QS, g, gq);
+  stk<NV, T>(d.grad, tp.grad, 0, QS, g, gq);
   for (; seq; seq &= seq - 1) limit_seq<T>(d, tp, g, __ffs(seq) - 1);
   // passive scalars: the same face-weighted slope and limiter
   for (int q = 5; q < 5 + (PS ? P.num_n : 0); ++q) {
@@ -740,7 +750,7 @@ __device__ __forceinline__ unsigned long long cfl_key(const DevPtrs &d, const An
   return key;
 }
 
-template <typename T, int MB = DGPU_MINB_PLM, bool PS = false>
+template <typename T, int MB = DGPU_MINB_PLM, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_plm_r(const __grid_constant__ DevPtrs d, const __grid_constant__ TanPtrs tp,
                                                                         int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -758,7 +768,8 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_plm_r(const __grid_
     }
   }
   if (g < N) {
-    plm_r_grad<T, PS>(d, tp, g);
+    if (V4 && no_vz(d)) plm_r_grad<T, PS, V4 ? 4 : 5>(d, tp, g);
+    else plm_r_grad<T, PS>(d, tp, g);
     const int a = d.cell_ann[g];
     const Annulus &A = d.ann[a];
     inst = A.inst;
@@ -800,15 +811,15 @@ __global__ void k_dt(DevPtrs d) {
 // ---------------------------------------------------------------------------
 // phi faces: thread per cell j, face (j, j+1) (riemann_setup_p, Riemann_setup.c:46-80)
 // ist: the disks' states with this substep's GravMass positions (NULL: d.ist).
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &tp, int g, const InstState *ist,
                                               int substep) {
   const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   // the cell's own planes (its right neighbour's share the lines) ahead of
   // the annulus lookups
-  pf_planes(d.prim, 5, QS, g);
-  pf_planes(d.gradp, 5, QS, g);
-  pf_planes(d.grad, 5, QS, g);
+  pf_planes(d.prim, NV, QS, g);
+  pf_planes(d.gradp, NV, QS, g);
+  pf_planes(d.grad, NV, QS, g);
   pf(d.tiphw + g);
   pf(d.dphi + g);
   const int a = d.cell_ann[g];
@@ -824,12 +835,12 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
   T pL[5], pR[5];
   {
     T gL[5], gR[5];
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, pL);
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, pR);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, gL);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, gR);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cL, pL);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cR, pR);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cL, gL);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cR, gR);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
+    for (int q = 0; q < NV; ++q) {
       pL[q] = pL[q] + 0.5 * gL[q] * dpL;
       pR[q] = pR[q] - 0.5 * gR[q] * dpR;
     }
@@ -842,17 +853,17 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
     qL[s] = ld(d.prim, 5 + s, QS, cL) + 0.5 * ld(d.gradp, 5 + s, QS, cL) * dpL;
     qR[s] = ld(d.prim, 5 + s, QS, cR) - 0.5 * ld(d.gradp, 5 + s, QS, cR) * dpR;
   }
-  riemann_flux(pL, pR, r, 1, w, P.gamma, P.riemann, F, np, qL, qR, Fq);
+  riemann_flux<NV>(pL, pR, r, 1, w, P.gamma, P.riemann, F, np, qL, qR, Fq);
   const InstState &S = ist ? *ist : d.ist[A.inst];
   const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) F[q] = k * F[q];
-  stk<5, T>(d.fphi, tp.fphi, 0, QF, g, F);
+  for (int q = 0; q < NV; ++q) F[q] = k * F[q];
+  stk<NV, T>(d.fphi, tp.fphi, 0, QF, g, F);
   for (int s = 0; s < np; ++s) d.fphi[ix(8 + s, QF, g)] = k * Fq[s];
   if (P.has_visc) {
     ViscIn<T> v;
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
     ldk<4, T>(d.grad, tp.grad, 0, QS, cL, v.grL);
     ldk<4, T>(d.grad, tp.grad, 0, QS, cR, v.grR);
     v.tL = d.tiphw[cL];
@@ -866,22 +877,23 @@ __device__ __forceinline__ void flux_phi_cell(const DevPtrs &d, const TanPtrs &t
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
     T Fv[3], u[4];
-    visc_flux(v, 1, P, G, Fv, d.err);
+    visc_flux<NV>(v, 1, P, G, Fv, d.err);
 #pragma unroll
     for (int q = 0; q < 3; ++q) u[1 + q] = k * Fv[q];
     stk<3, T>(d.fphi, tp.fphi, 5, QF, g, u + 1);
   }
 }
 
-template <typename T, int MB = DGPU_MINB_FLUX, bool PS = false>
+template <typename T, int MB = DGPU_MINB_FLUX, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_flux_phi(DevPtrs d, TanPtrs tp, int substep) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.n_cells) return;
-  flux_phi_cell<T, PS>(d, tp, g, nullptr, substep);
+  if (V4 && no_vz(d)) flux_phi_cell<T, PS, V4 ? 4 : 5>(d, tp, g, nullptr, substep);
+  else flux_phi_cell<T, PS>(d, tp, g, nullptr, substep);
 }
 
 // r faces: thread per face slot (riemann_setup_rz, Riemann_setup.c:11-44)
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp, int slot, const InstState *ist,
                                             int substep) {
   const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
@@ -903,16 +915,16 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
   T pL[5], pR[5];
   {
     T u[5], w[5];
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, pL);
-    ldk<5, T>(d.grad, tp.grad, 0, QS, cL, u);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, w);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cL, pL);
+    ldk<NV, T>(d.grad, tp.grad, 0, QS, cL, u);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cL, w);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) pL[q] = pL[q] + u[q] * deltaL + w[q] * dpL;
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, pR);
-    ldk<5, T>(d.grad, tp.grad, 0, QS, cR, u);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, w);
+    for (int q = 0; q < NV; ++q) pL[q] = pL[q] + u[q] * deltaL + w[q] * dpL;
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cR, pR);
+    ldk<NV, T>(d.grad, tp.grad, 0, QS, cR, u);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cR, w);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) pR[q] = pR[q] - u[q] * deltaR - w[q] * dpR;
+    for (int q = 0; q < NV; ++q) pR[q] = pR[q] - u[q] * deltaR - w[q] * dpR;
   }
   T F[5];
   double qL[DGPU_MAX_PASSIVE], qR[DGPU_MAX_PASSIVE], Fq[DGPU_MAX_PASSIVE];
@@ -921,19 +933,19 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
     qL[s] = ld(d.prim, 5 + s, QS, cL) + ld(d.grad, 5 + s, QS, cL) * deltaL + ld(d.gradp, 5 + s, QS, cL) * dpL;
     qR[s] = ld(d.prim, 5 + s, QS, cR) - ld(d.grad, 5 + s, QS, cR) * deltaR - ld(d.gradp, 5 + s, QS, cR) * dpR;
   }
-  riemann_flux(pL, pR, r, 0, 0.0, P.gamma, P.riemann, F, np, qL, qR, Fq);
+  riemann_flux<NV>(pL, pR, r, 0, 0.0, P.gamma, P.riemann, F, np, qL, qR, Fq);
   const InstState &S = ist ? *ist : d.ist[A.inst];
   const double k = (substep == 1 ? 1.0 : 0.5) * step_dt(d, S, P, substep) * dA;
 #pragma unroll
-  for (int q = 0; q < 5; ++q) F[q] = k * F[q];
-  stk<5, T>(d.frf, tp.frf, 0, QF, slot, F);
+  for (int q = 0; q < NV; ++q) F[q] = k * F[q];
+  stk<NV, T>(d.frf, tp.frf, 0, QF, slot, F);
   for (int s = 0; s < np; ++s) d.frf[ix(8 + s, QF, slot)] = k * Fq[s];
   if (P.has_visc) {
     ViscIn<T> v;
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
-    ldk<5, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cL, v.gpL);
-    ldk<5, T>(d.gradp, tp.gradp, 0, QS, cR, v.gpR);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cL, v.cL);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, cR, v.cR);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cL, v.gpL);
+    ldk<NV, T>(d.gradp, tp.gradp, 0, QS, cR, v.gpR);
     v.tL = d.tiphw[cL];
     v.tR = d.tiphw[cR];
     v.dpL = dpL;
@@ -946,18 +958,19 @@ __device__ __forceinline__ void flux_r_face(const DevPtrs &d, const TanPtrs &tp,
     GravT<T> G;
     grav_t(G, S, P, tp, A.inst);
     T Fv[3], u[4];
-    visc_flux(v, 0, P, G, Fv, d.err);
+    visc_flux<NV>(v, 0, P, G, Fv, d.err);
 #pragma unroll
     for (int q = 0; q < 3; ++q) u[1 + q] = k * Fv[q];
     stk<3, T>(d.frf, tp.frf, 5, QF, slot, u + 1);
   }
 }
 
-template <typename T, int MB = DGPU_MINB_FLUXR, bool PS = false>
+template <typename T, int MB = DGPU_MINB_FLUXR, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_flux_r(DevPtrs d, TanPtrs tp, int substep) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= d.n_slots) return;
-  flux_r_face<T, PS>(d, tp, slot, nullptr, substep);
+  if (V4 && no_vz(d)) flux_r_face<T, PS, V4 ? 4 : 5>(d, tp, slot, nullptr, substep);
+  else flux_r_face<T, PS>(d, tp, slot, nullptr, substep);
 }
 
 // ---------------------------------------------------------------------------
@@ -1167,12 +1180,12 @@ __device__ __forceinline__ void ann_consts(const DevPtrs &d, int t, const InstSt
 
 // The source increments of cell g (see k_source); the sink masses of the
 // cells counted in Mdot are added to md0 / md1.
-template <typename T, bool PS>
+template <typename T, bool PS, int NV = 5>
 __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &tp, int g, const InstState &S,
                                               double dt, double &md0, double &md1) {
   const Pl QS = {PS ? d.qs : 5};
   {
-    pf_planes(d.prim, 5, QS, g);
+    pf_planes(d.prim, NV, QS, g);
     pf(d.grad + ix(D_UPP, QS, g));
     pf(d.gradp + ix(D_URR, QS, g));
     pf(d.tiphw + g);
@@ -1185,7 +1198,7 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
     double phi = d.tiphw[g] - .5 * dphi;
     double r = .5 * (rp + rm);
     T pm[5];
-    ldk<5, T>(d.prim, tp.prim, 0, QS, g, pm);
+    ldk<NV, T>(d.prim, tp.prim, 0, QS, g, pm);
     SrcGeom sg;
     sg.r = r;
     sg.dt = dt;
@@ -1220,8 +1233,10 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
       gpu = ldq<T>(d.gradp, tp.gradp, D_URR, QS, g);
     }
     T sv[6];
-    source_cell(sg, P, pm, gu, gpu, G, sv);
-    stk<6, T>(d.src, tp.src, 0, P8, g, sv);
+    source_cell<NV>(sg, P, pm, gu, gpu, G, sv);
+    stk<3, T>(d.src, tp.src, 0, P8, g, sv);
+    if constexpr (NV == 5) stq<T>(d.src, tp.src, 3, P8, g, sv[3]);
+    stk<2, T>(d.src, tp.src, 4, P8, g, sv + 4);
     const double xpos = sg.xpos, ypos = sg.ypos, dV = sg.dV;
     const T rho = pm[D_RHO], Pp = pm[D_PPP];
     if (P.rho_sink_on == 1) {
@@ -1253,7 +1268,7 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
   }
 }
 
-template <typename T, int MB = DGPU_MINB_SOURCE, bool PS = false>
+template <typename T, int MB = DGPU_MINB_SOURCE, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int substep, int cells) {
   __shared__ double sh_md[2][BLK / 32];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1268,7 +1283,9 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
   if (t < N && cells) {
     const int inst = d.ann[d.cell_ann[t]].inst;
     const InstState &S = d.ist[inst];
-    source_cell_k<T, PS>(d, tp, t, S, fac * step_dt(d, S, d.par[inst], substep), md0, md1);
+    const double dt = fac * step_dt(d, S, d.par[inst], substep);
+    if (V4 && no_vz(d)) source_cell_k<T, PS, V4 ? 4 : 5>(d, tp, t, S, dt, md0, md1);
+    else source_cell_k<T, PS>(d, tp, t, S, dt, md0, md1);
   }
   // deterministic per-block Mdot partial sums (reduced in block order by k_update)
   const unsigned full = 0xffffffffu;
@@ -1301,15 +1318,15 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
 // not the read-only path).  rec (the adjoint's segment replay, else NULL): the
 // conserved sum before cons2prim and the new width of each cell go to slot
 // 2 * (*rec_idx) + substep - 1 of rec (per slot 6 planes over n_pad cells).
-template <typename T, bool PS, bool XC = false>
+template <typename T, bool PS, bool XC = false, int NV = 5>
 __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp, int g, int substep, int stop,
                                             const InstState *ist, double *rec, const int *rec_idx) {
   const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
   {
     // the cell's own planes, before the annulus lookups they do not depend on
-    pf_planes(d.cons, 5, QS, g);
+    pf_planes(d.cons, NV, QS, g);
     if (substep == 2) {
-      pf_planes(d.rkcons, 5, QS, g);
+      pf_planes(d.rkcons, NV, QS, g);
       pf(d.rktiph + g);
     }
     pf_planes(d.fphi, 8, QF, g);
@@ -1327,8 +1344,8 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
     double cp[DGPU_MAX_PASSIVE], pp[DGPU_MAX_PASSIVE];
     const int np = PS ? P.num_n : 0;
     if (np > 0) passive_sum(d, A, a, g, substep, stop, np, cp);
-    if (!update_sum<T, !XC, PS>(d, tp, A, a, g, substep, stop, dt, true, c)) {
-      stk<5, T>(d.cons, tp.cons, 0, QS, g, c);
+    if (!update_sum<T, !XC, PS, NV>(d, tp, A, a, g, substep, stop, dt, true, c)) {
+      stk<NV, T>(d.cons, tp.cons, 0, QS, g, c);
       for (int k = 0; k < np; ++k) d.cons[ix(5 + k, QS, g)] = cp[k];
     } else {
       double tn, rk;
@@ -1339,8 +1356,9 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       if (rec) {
         double *rs = rec + (size_t)(2 * (*rec_idx) + substep - 1) * 6 * d.n_pad;
         double u[6];
+        u[D_SZZ] = 0.0;
 #pragma unroll
-        for (int q = 0; q < 5; ++q) u[q] = val(c[q]);
+        for (int q = 0; q < NV; ++q) u[q] = val(c[q]);
         u[5] = dphi_n;
         stk<6>(rs, 0, P6, g, u);
       }
@@ -1348,19 +1366,20 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       const double r = .5 * (A.rm + A.rp);
       const double dV = A.dv_half * dphi_n * A.dz;
       T pr[5];
-      cons2prim(c, dV, r, P, pr);
+      cons2prim<NV>(c, dV, r, P, pr);
       // passive scalars: prim = cons / cons[DDD] (cell_conversion.c:98-101)
       for (int k = 0; k < np; ++k) pp[k] = cp[k] / val(c[D_DDD]);
       // the outflow boundary reads these prims before any damping; the
       // annuli it rewrites are damped and converted by k_outflow
       if (A.ob_off >= 0 && stop >= 6) {
 #pragma unroll
-        for (int q = 0; q < 5; ++q) d.obuf[(size_t)q * d.n_ob + A.ob_off + (g - A.cell_off)] = val(pr[q]);
+        for (int q = 0; q < 5; ++q)
+          d.obuf[(size_t)q * d.n_ob + A.ob_off + (g - A.cell_off)] = q < NV ? val(pr[q]) : 0.0;
         for (int k = 0; k < np; ++k) d.obuf[(size_t)(5 + k) * d.n_ob + A.ob_off + (g - A.cell_off)] = pp[k];
       }
       const bool own = !(A.kind & DGPU_AK_OUT_DST);
       if (stop >= 6 && own) {
-        bc_damp(d, A, a, pr);
+        bc_damp<NV>(d, A, a, pr);
         // cell_single_init_vortex's dye at the cell's new phi, in the fixed
         // boundary (cell_init_vortex.c:22-35); no other family sets one
         if (np > 0 && P.init_type == DI_VORTEX && (A.kind & DGPU_AK_BC_FIXED) && (A.kind & DGPU_AK_IC))
@@ -1368,11 +1387,11 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       }
       // cell_calc_cons (src/Cell/cell_conversion.c:35-55)
       if (stop >= 7 && own) {
-        prim2cons(pr, c, r, dV, P.gamma);
+        prim2cons<NV>(pr, c, r, dV, P.gamma);
         for (int k = 0; k < np; ++k) cp[k] = pp[k] * val(c[D_DDD]);
       }
-      stk<5, T>(d.prim, tp.prim, 0, QS, g, pr);
-      stk<5, T>(d.cons, tp.cons, 0, QS, g, c);
+      stk<NV, T>(d.prim, tp.prim, 0, QS, g, pr);
+      stk<NV, T>(d.cons, tp.cons, 0, QS, g, c);
       for (int k = 0; k < np; ++k) {
         d.prim[ix(5 + k, QS, g)] = pp[k];
         d.cons[ix(5 + k, QS, g)] = cp[k];
@@ -1435,7 +1454,7 @@ __device__ __forceinline__ void gm_tail(const DevPtrs &d, InstState &S, const Di
 // disk instead, while the others work: no cell of this kernel reads what it
 // writes.  (A last block elected by a counter did it after all the others, a
 // chain of two pow at the end of every substep.)
-template <typename T, int MB = DGPU_MINB_UPDATE, bool PS = false>
+template <typename T, int MB = DGPU_MINB_UPDATE, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, TanPtrs tp, int substep, int stop,
                                                                   int tail, double *rec, const int *rec_idx) {
   int b = blockIdx.x;
@@ -1462,7 +1481,8 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, T
   }
   const int g = b * TBLK + threadIdx.x;
   if (g >= d.n_cells) return;
-  update_cell<T, PS>(d, tp, g, substep, stop, nullptr, rec, rec_idx);
+  if (V4 && no_vz(d)) update_cell<T, PS, false, V4 ? 4 : 5>(d, tp, g, substep, stop, nullptr, rec, rec_idx);
+  else update_cell<T, PS>(d, tp, g, substep, stop, nullptr, rec, rec_idx);
 }
 
 // ---------------------------------------------------------------------------
@@ -1948,10 +1968,22 @@ __global__ void __launch_bounds__(BLK) k_torque(DevPtrs d, int inst, double *par
 
 // AoS rows [n][nq] (the boundary format) <-> cells base .. base + n of an
 // array of `planes` planes
-__global__ void k_aos_to_soa(double *soa, int nq, Pl planes, int base, const double *aos, int n) {
+// vz (may be NULL): set when a row has a v_z
+__global__ void k_aos_to_soa(double *soa, int nq, Pl planes, int base, const double *aos, int n, int *vz) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
+  if (vz && aos[(size_t)c * nq + D_UZZ] != 0.0) *vz = 1;
   for (int q = 0; q < nq; ++q) soa[ix(q, planes, base + c)] = aos[(size_t)c * nq + q];
+}
+// The context's v_z flag vz[0] from the disks' vz[1 + k].
+__global__ void k_any_vz(int *vz, int n_inst) {
+  __shared__ int any;
+  if (threadIdx.x == 0) any = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < n_inst; k += blockDim.x)
+    if (vz[1 + k]) any = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) vz[0] = any;
 }
 __global__ void k_soa_to_aos(double *aos, int nq, Pl planes, int base, const double *soa, int n) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1963,9 +1995,13 @@ __global__ void k_soa_to_aos(double *aos, int nq, Pl planes, int base, const dou
 
 extern "C" {
 
-int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, void *stream) {
+int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, int *vz, void *stream) {
   if (n <= 0) return 0;
-  k_aos_to_soa<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(soa, nq, Pl{planes}, base, aos, n);
+  k_aos_to_soa<<<(n + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(soa, nq, Pl{planes}, base, aos, n, vz);
+  return (int)cudaGetLastError();
+}
+int dgk_any_vz(int *vz, int n_inst, void *stream) {
+  k_any_vz<<<1, BLK, 0, (cudaStream_t)stream>>>(vz, n_inst);
   return (int)cudaGetLastError();
 }
 int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream) {
@@ -1977,6 +2013,9 @@ int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa,
 int dgk_update_blocks(int n_cells) { return (n_cells + BLK - 1) / BLK; }
 int dgk_block_size(void) { return BLK; }
 
+// Whether the context's disks can be without a v_z at all.
+static bool may_v4(const DevPtrs *d) { return d->vz && !d->has_z; }
+
 // t == NULL: the forward kernels; otherwise their tangent instances.
 // Contexts with passive scalars take the instances that carry them (PS).
 #define DGK_LAUNCH(kern, grid, smem, stream, ...)                                                  \
@@ -1985,12 +2024,22 @@ int dgk_block_size(void) { return BLK; }
     if (t) kern<Dual><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, *t, __VA_ARGS__);       \
     else if (d->n_pass > 0)                                                                       \
       kern<double, true><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, none_, __VA_ARGS__); \
+    else if (!may_v4(d))                                                                          \
+      kern<double, false, false><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, none_, __VA_ARGS__); \
     else kern<double><<<(grid), BLK, (smem), (cudaStream_t)(stream)>>>(*d, none_, __VA_ARGS__);    \
   } while (0)
 // The same for the kernels the autotuner sizes, in blocks of blk threads: the
 // forward instance with d->tune[which] resident blocks of BLK threads per SM
 // (0: the built-in choice).
-#define DGK_LAUNCH_TUNED(kern, which, mbdef, grid, blk, stream, ...)                           \
+#define DGK_TUNE_SWITCH(kern, which, mbdef, v4, grid, blk, s_, ...)                              \
+  switch (d->tune[which]) {                                                                     \
+    case 2: kern<double, 2, false, v4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+    case 3: kern<double, 3, false, v4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+    case 4: kern<double, 4, false, v4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+    case 5: kern<double, 5, false, v4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
+    default: kern<double, mbdef, false, v4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__);    \
+  }
+#define DGK_LAUNCH_TUNED(kern, which, mbdef, grid, blk, stream, ...)                      \
   do {                                                                                   \
     static const TanPtrs none_ = {};                                                     \
     cudaStream_t s_ = (cudaStream_t)(stream);                                            \
@@ -1998,14 +2047,10 @@ int dgk_block_size(void) { return BLK; }
       kern<Dual><<<(grid), blk, 0, s_>>>(*d, *t, __VA_ARGS__);                            \
     } else if (d->n_pass > 0) {                                                          \
       kern<double, mbdef, true><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__);          \
+    } else if (may_v4(d)) {                                                              \
+      DGK_TUNE_SWITCH(kern, which, mbdef, true, grid, blk, s_, __VA_ARGS__)              \
     } else {                                                                             \
-      switch (d->tune[which]) {                                                          \
-        case 2: kern<double, 2><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 3: kern<double, 3><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 4: kern<double, 4><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        case 5: kern<double, 5><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__); break;   \
-        default: kern<double><<<(grid), blk, 0, s_>>>(*d, none_, __VA_ARGS__);           \
-      }                                                                                  \
+      DGK_TUNE_SWITCH(kern, which, mbdef, false, grid, blk, s_, __VA_ARGS__)             \
     }                                                                                    \
   } while (0)
 
@@ -2022,6 +2067,7 @@ int dgk_rslope(const DevPtrs *d, const TanPtrs *t, void *stream) {
   static const TanPtrs none = {};
   if (t) k_rslope<Dual><<<(d->n_slots + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, *t);
   else if (d->n_pass > 0) k_rslope<double, true><<<(d->n_slots + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, none);
+  else if (!may_v4(d)) k_rslope<double, false, false><<<(d->n_slots + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, none);
   else k_rslope<double><<<(d->n_slots + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, none);
   return (int)cudaGetLastError();
 }
@@ -2060,12 +2106,12 @@ int dgk_update(const DevPtrs *d, const TanPtrs *t, int substep, int stop, void *
 }
 int dgk_update_rec(const DevPtrs *d, int substep, double *rec, const int *rec_idx, void *stream) {
   static const TanPtrs none = {};
-  k_update<double><<<update_grid(d, 2), TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 7, 2, rec, rec_idx);
+  k_update<double, DGPU_MINB_UPDATE, false, false><<<update_grid(d, 2), TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 7, 2, rec, rec_idx);
   return (int)cudaGetLastError();
 }
 int dgk_ann_consts(const DevPtrs *d, int substep, void *stream) {
   static const TanPtrs none = {};
-  k_source<double><<<(d->n_ann + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 0);
+  k_source<double, DGPU_MINB_SOURCE, false, false><<<(d->n_ann + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d, none, substep, 0);
   return (int)cudaGetLastError();
 }
 int dgk_update_stage(const DevPtrs *d, int substep, int stop, void *stream) {
@@ -2076,7 +2122,7 @@ int dgk_update_stage(const DevPtrs *d, int substep, int stop, void *stream) {
     k_update<double, DGPU_MINB_UPDATE, true><<<nb, TBLK, 0, (cudaStream_t)stream>>>(
         *d, none, substep, stop, tail, nullptr, nullptr);
   else
-    k_update<double><<<nb, TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, stop, tail, nullptr, nullptr);
+    k_update<double, DGPU_MINB_UPDATE, false, false><<<nb, TBLK, 0, (cudaStream_t)stream>>>(*d, none, substep, stop, tail, nullptr, nullptr);
   return (int)cudaGetLastError();
 }
 int dgk_zmerge(const DevPtrs *d, int substep, void *stream) {

@@ -35,6 +35,13 @@ __device__ __forceinline__ void grav_t(GravT<T> &G, const InstState &S, const Di
   }
 }
 
+// No disk of the context has a v_z: 2-D disks whose prims were set with
+// v_z = 0 and whose gravity has no vertical part keep it 0 (every term of its
+// flux and source is a product with 0).  The step's kernels then leave out
+// plane UZZ / SZZ, a fifth of the state's traffic and about a tenth of the
+// arithmetic.  d.vz is set by the uploads; NULL: always all planes.
+__device__ __forceinline__ bool no_vz(const DevPtrs &d) { return d.vz && rd(d.vz) == 0; }
+
 // timestep_set_dt (timestep_set.c:16-21): the CFL minimum that k_plm_r left in
 // dtkey, clipped to Time_Max.
 __device__ __forceinline__ double cfl_dt(const InstState &S, const DiskParams &P) {
@@ -75,7 +82,7 @@ __device__ __forceinline__ double new_tiph(double tw, double &rk, double RK, dou
 // Writes rkcons in substep 1 when `write_rk`.  NC: the increments and the
 // annulus constants come from earlier kernels (the read-only path), not from
 // another block of the running one (plain loads).
-template <typename T, bool NC = true, bool PS = false>
+template <typename T, bool NC = true, bool PS = false, int NV = 5>
 __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, const Annulus &A, int a, int g,
                                            int substep, int stop, double dt, bool write_rk, T *c) {
   const Pl QS = {PS ? d.qs : 5}, QF = {PS ? d.qf : 8};
@@ -86,29 +93,32 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   // cell_copy (substep 1) + cell_adjust_RK_cons (cell_misc.c:28-57)
   {
     T rk[5];
-    ldk<5, T, true>(d.cons, tp.cons, 0, QS, g, c);
+    ldk<NV, T, true>(d.cons, tp.cons, 0, QS, g, c);
     if (substep == 1) {
 #pragma unroll
-      for (int q = 0; q < 5; ++q) rk[q] = c[q];
-      if (write_rk) stk<5, T>(d.rkcons, tp.rkcons, 0, QS, g, c);
+      for (int q = 0; q < NV; ++q) rk[q] = c[q];
+      if (write_rk) stk<NV, T>(d.rkcons, tp.rkcons, 0, QS, g, c);
     } else {
-      ldk<5, T, true>(d.rkcons, tp.rkcons, 0, QS, g, rk);
+      ldk<NV, T, true>(d.rkcons, tp.rkcons, 0, QS, g, rk);
     }
 #pragma unroll
-    for (int q = 0; q < 5; ++q) c[q] = (1.0 - RK) * c[q] + RK * rk[q];
+    for (int q = 0; q < NV; ++q) c[q] = (1.0 - RK) * c[q] + RK * rk[q];
   }
   if (stop <= 1) return false;
   // phi faces: for j = 0 the face (0,1) comes before (N-1,0)
   {
     const int gl = j == 0 ? A.cell_off + np - 1 : g - 1;
     const double r = .5 * (A.rp + A.rm);
-    // the eight increments of a face, the viscous ones after the others
+    // the increments of a face, the viscous ones (5 to 7) after the others
+    auto load = [&](int f, T *u) {
+      ldk<NV, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
+      if (P.has_visc) ldk<3, T, NC>(d.fphi, tp.fphi, 5, QF, f, u + 5);
+    };
     auto addL = [&](int f) {
       T u[8];
-      if (P.has_visc) ldk<8, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
-      else ldk<5, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
+      load(f, u);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) c[q] -= u[q];
+      for (int q = 0; q < NV; ++q) c[q] -= u[q];
       if (P.has_visc) {
         c[D_SRR] -= u[5] / r;
         c[D_LLL] -= u[6];
@@ -117,10 +127,9 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
     };
     auto addR = [&](int f) {
       T u[8];
-      if (P.has_visc) ldk<8, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
-      else ldk<5, T, NC>(d.fphi, tp.fphi, 0, QF, f, u);
+      load(f, u);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) c[q] += u[q];
+      for (int q = 0; q < NV; ++q) c[q] += u[q];
       if (P.has_visc) {
         c[D_SRR] += u[5] / r;
         c[D_LLL] += u[6];
@@ -147,7 +156,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
       auto apply = [&](const T *u) {
         if (asR) {
 #pragma unroll
-          for (int q = 0; q < 5; ++q) c[q] += u[q];
+          for (int q = 0; q < NV; ++q) c[q] += u[q];
           if (visc) {
             c[D_SRR] += u[5] / rv;
             c[D_LLL] += u[6];
@@ -155,7 +164,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
           }
         } else {
 #pragma unroll
-          for (int q = 0; q < 5; ++q) c[q] -= u[q];
+          for (int q = 0; q < NV; ++q) c[q] -= u[q];
           if (visc) {
             c[D_SRR] -= u[5] / rv;
             c[D_LLL] -= u[6];
@@ -165,8 +174,8 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
       };
       for (int n = s; n < e; ++n) {
         T u[8];
-        if (visc) ldk<8, T, NC>(d.frf, tp.frf, 0, QF, n, u);
-        else ldk<5, T, NC>(d.frf, tp.frf, 0, QF, n, u);
+        ldk<NV, T, NC>(d.frf, tp.frf, 0, QF, n, u);
+        if (visc) ldk<3, T, NC>(d.frf, tp.frf, 5, QF, n, u + 5);
         apply(u);
       }
     });
@@ -175,7 +184,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   // increments of pair (a-NR, a) are added, those of (a, a+NR) subtracted.  Their
   // viscous flux is zero (riemann_visc_flux sets neither the r nor the phi
   // terms); adding its +0 to the upper cell keeps the reference's signed zeros.
-  if constexpr (std::is_same<T, double>::value) {
+  if constexpr (std::is_same<T, double>::value && NV == 5) {
     if (d.has_z && P.NZ > 1) {
       const bool visc = P.has_visc;
       for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int up) {
@@ -184,7 +193,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
           ldk<5, NC>(d.zfrf, 0, P5, n, u);
           if (up) {
 #pragma unroll
-            for (int q = 0; q < 5; ++q) c[q] += u[q];
+            for (int q = 0; q < NV; ++q) c[q] += u[q];
             if (visc) {
               c[D_SRR] += 0.0;
               c[D_LLL] += 0.0;
@@ -192,7 +201,7 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
             }
           } else {
 #pragma unroll
-            for (int q = 0; q < 5; ++q) c[q] -= u[q];
+            for (int q = 0; q < NV; ++q) c[q] -= u[q];
           }
         }
       });
@@ -202,11 +211,13 @@ __device__ __forceinline__ bool update_sum(const DevPtrs &d, const TanPtrs &tp, 
   // cell_add_src, cell_add_visc_src, cell_add_split_fictitious: the source
   // increments come from k_source; added here in the reference's order
   T u[6];
-  ldk<6, T, NC>(d.src, tp.src, 0, P8, g, u);
+  ldk<3, T, NC>(d.src, tp.src, 0, P8, g, u);
+  if constexpr (NV == 5) u[3] = NC ? ldqr<T>(d.src, tp.src, 3, P8, g) : ldq<T>(d.src, tp.src, 3, P8, g);
+  ldk<2, T, NC>(d.src, tp.src, 4, P8, g, u + 4);
   c[D_SRR] += u[0];
   c[D_SRR] += u[1];
   c[D_LLL] += u[2];
-  c[D_SZZ] += u[3];
+  if constexpr (NV == 5) c[D_SZZ] += u[3];
   c[D_TAU] += u[4];
   if (P.rho_sink_on == 1) {
     for (int p = 0; p < P.num_sinks && p < 2; ++p)
@@ -310,17 +321,17 @@ __device__ __forceinline__ double mesh_advance(const DevPtrs &d, const Annulus &
 
 // cell_boundary_fixed_r (src/Cell/cell_boundary.c:208-231) and cell_bc_damp
 // (src/Cell/cell_misc.c:98-132) on the new prims of a cell.
-template <typename T>
+template <int NV = 5, typename T>
 __device__ __forceinline__ void bc_damp(const DevPtrs &d, const Annulus &A, int a, T *pr) {
   const DiskParams &P = d.par[A.inst];
   if ((A.kind & DGPU_AK_BC_FIXED) && (A.kind & DGPU_AK_IC)) {
 #pragma unroll
-    for (int q = 0; q < 5; ++q) pr[q] = A.ic[q];
+    for (int q = 0; q < NV; ++q) pr[q] = A.ic[q];
   }
   if (P.has_damp && (A.kind & DGPU_AK_DAMP) && (A.kind & DGPU_AK_IC)) {
     double f = d.ann_c[3 * d.n_ann + a];  // 1.-exp(-rate*dt), k_source
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
+    for (int q = 0; q < NV; ++q) {
       T dprim = A.ic[q] - pr[q];
       pr[q] += f * dprim;
     }
