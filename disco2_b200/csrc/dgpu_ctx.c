@@ -832,11 +832,14 @@ int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub) {
 static int launch_substep_3d(struct dgpu_ctx *c, int sub) {
   CK(cudaEventRecord(c->fork[0], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[0], 0));
+  CK(cudaStreamWaitEvent(c->side2, c->fork[0], 0));
   CKK(dgk_merge(&c->d, sub, c->side));
-  CKK(dgk_zmerge(&c->d, sub, c->side));
+  CKK(dgk_zmerge(&c->d, sub, c->side2));
   CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
   CK(cudaEventRecord(c->fork[1], c->side));
   CK(cudaStreamWaitEvent(c->stream, c->fork[1], 0));
+  CK(cudaEventRecord(c->fork[4], c->side2));
+  CK(cudaStreamWaitEvent(c->stream, c->fork[4], 0));
   CK(cudaEventRecord(c->fork[2], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[2], 0));
   CKK(dgk_zslope(&c->d, c->side));
