@@ -476,7 +476,8 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
       if (m > mx) mx = m;
       if (mz > mx) mx = mz;
     }
-    c->d.smem_face = mx <= 48 * 1024 ? mx : 0;
+    /* (with the kernel's own static arrays within 48 KB) */
+    c->d.smem_face = mx <= 46 * 1024 ? mx : 0;
   }
   {
     /* threads per merge block: 256, or fewer when every annulus is small, so
