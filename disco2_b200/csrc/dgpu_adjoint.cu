@@ -827,15 +827,23 @@ int dgk_adj_rows(const DevPtrs *d) {
   return 3 * nbC + nbS;
 }
 
+/* The sums over the partial rows (a_par_reduce, one block) run on the side
+ * stream: nothing but J.acc and the next use of the rows waits for them. */
 int dgk_adj_objective(const DevPtrs *d, const AdjPtrs *J, double *const *bufs, InstState *const *ists,
-                      const int *idx, int off, const double *wts, const int *base, void *stream) {
+                      const int *idx, int off, const double *wts, const int *base, void *stream, void *side,
+                      void *ev) {
+  cudaStream_t s = (cudaStream_t)stream, s2 = (cudaStream_t)side;
   const int nbC = (d->n_cells + BLK - 1) / BLK, nbS = (d->n_slots + BLK - 1) / BLK;
   const int row0 = 2 * nbC + nbS;
-  a_objective<<<nbC, BLK, 0, (cudaStream_t)stream>>>(*d, *J, bufs, ists, idx, off, wts, base, row0);
-  a_par_reduce<<<1, BLK, 0, (cudaStream_t)stream>>>(*J, row0, nbC);
+  cudaError_t e;
+  a_objective<<<nbC, BLK, 0, s>>>(*d, *J, bufs, ists, idx, off, wts, base, row0);
+  if ((e = cudaEventRecord((cudaEvent_t)ev, s)) != cudaSuccess) return (int)e;
+  if ((e = cudaStreamWaitEvent(s2, (cudaEvent_t)ev, 0)) != cudaSuccess) return (int)e;
+  a_par_reduce<<<1, BLK, 0, s2>>>(*J, row0, nbC);
   return (int)cudaGetLastError();
 }
 
+/* The side stream joins at the end. */
 int dgk_adj_substep(const DevPtrs *d, const AdjPtrs *J, int substep, const double *rec, const int *idx,
                     void *stream, void *side, void *ev_fork, void *ev_join) {
   cudaStream_t s = (cudaStream_t)stream, s2 = (cudaStream_t)side;
@@ -848,11 +856,15 @@ int dgk_adj_substep(const DevPtrs *d, const AdjPtrs *J, int substep, const doubl
   a_flux_phi<<<nbC, BLK, 0, s2>>>(*d, *J, substep, nbC);
   if (nbS > 0) a_flux_r<<<nbS, BLK, 0, s>>>(*d, *J, substep, 2 * nbC);
   if ((e = cudaEventRecord((cudaEvent_t)ev_join, s2)) != cudaSuccess) return (int)e;
+  if ((e = cudaEventRecord((cudaEvent_t)ev_fork, s)) != cudaSuccess) return (int)e;
   if ((e = cudaStreamWaitEvent(s, (cudaEvent_t)ev_join, 0)) != cudaSuccess) return (int)e;
-  a_par_reduce<<<1, BLK, 0, s>>>(*J, 0, 2 * nbC + nbS);
+  if ((e = cudaStreamWaitEvent(s2, (cudaEvent_t)ev_fork, 0)) != cudaSuccess) return (int)e;
+  a_par_reduce<<<1, BLK, 0, s2>>>(*J, 0, 2 * nbC + nbS);
   a_gather_plm<<<nbC, BLK, 0, s>>>(*d, *J);
   a_rslope<<<nbC, BLK, 0, s>>>(*d, *J);
   a_cellprep<<<nbC, BLK, 0, s>>>(*d, *J);
+  if ((e = cudaEventRecord((cudaEvent_t)ev_join, s2)) != cudaSuccess) return (int)e;
+  if ((e = cudaStreamWaitEvent(s, (cudaEvent_t)ev_join, 0)) != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }
 

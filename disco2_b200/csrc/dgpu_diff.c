@@ -491,7 +491,9 @@ static int record_graph(struct dgpu_ctx *c, struct dgpu_diff *D, int which) {
                          (stream s3; at *idx = 0 the slot is clamped to 0 and the
                          rebuild goes unused) */
       DevPtrs *b2 = &Dd->rb[par], *b1 = &Dd->rb[2 + par], *n2 = &Dd->rb[1 - par], *n1 = &Dd->rb[3 - par];
-      if (dgk_adj_objective(&c->d, &Dd->J, tabS, istS, Dd->d_idx, 1, Dd->wts, Dd->d_base, c->stream)) return -1;
+      if (dgk_adj_objective(&c->d, &Dd->J, tabS, istS, Dd->d_idx, 1, Dd->wts, Dd->d_base, c->stream, c->side,
+                            c->fork[0]))
+        return -1;
       if (cudaEventRecord(Dd->e_fork, c->stream) != cudaSuccess ||
           cudaStreamWaitEvent(Dd->s3, Dd->e_fork, 0) != cudaSuccess)
         return -1;

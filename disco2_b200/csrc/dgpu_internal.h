@@ -307,7 +307,7 @@ int dgk_snap_tab(const DevPtrs *d, double *const *bufs, InstState *const *ists, 
                  void *stream);
 int dgk_adj_rows(const DevPtrs *d);
 int dgk_adj_objective(const DevPtrs *d, const AdjPtrs *J, double *const *bufs, InstState *const *ists,
-                      const int *idx, int off, const double *wts, const int *base, void *stream);
+                      const int *idx, int off, const double *wts, const int *base, void *stream, void *side, void *ev);
 int dgk_adj_substep(const DevPtrs *d, const AdjPtrs *J, int substep, const double *rec, const int *idx,
                     void *stream, void *side, void *ev_fork, void *ev_join);
 int dgk_adj_calc_cons(const DevPtrs *d, const AdjPtrs *J, void *stream);
