@@ -477,7 +477,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
       if (mz > mx) mx = mz;
     }
     /* (with the kernel's own static arrays within 48 KB) */
-    c->d.smem_face = mx <= 46 * 1024 ? mx : 0;
+    c->d.smem_face = mx <= 44 * 1024 ? mx : 0;
   }
   {
     /* threads per merge block: 256, or fewer when every annulus is small, so
@@ -499,6 +499,9 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
     if (c->h_par[k].rho_sink_on == 1) c->fused_ok = 0;
   c->fused = 0;
   c->d.form_dt = few_waves(c);
+  c->d.has_rigid = 0;
+  for (k = 0; k < n; ++k)
+    if (c->h_par[k].w_numeric == DC_RIGID) c->d.has_rigid = 1;
   c->d.n_inst = n;
   c->d.n_ann = c->n_ann;
   c->d.n_cells = c->n_cells;
@@ -800,9 +803,17 @@ int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub) {
   CK(cudaEventRecord(c->fork[0], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[0], 0));
   CKK(dgk_merge(&c->d, sub, c->side));
+  if (c->d.has_rigid) {
+    CK(cudaStreamWaitEvent(c->side2, c->fork[0], 0));
+    CKK(dgk_ring_mean(&c->d, c->side2));
+  }
   CKK(dgk_cellprep(&c->d, t, sub, c->stream));
   CK(cudaEventRecord(c->fork[1], c->side));
   CK(cudaStreamWaitEvent(c->stream, c->fork[1], 0));
+  if (c->d.has_rigid) {
+    CK(cudaEventRecord(c->fork[4], c->side2));
+    CK(cudaStreamWaitEvent(c->stream, c->fork[4], 0));
+  }
   CKK(dgk_rslope(&c->d, t, c->stream));
   CKK(dgk_plm_r(&c->d, t, sub, c->stream));
   if (sub == 1 && !c->d.form_dt) CKK(dgk_dt(&c->d, c->stream));
@@ -836,6 +847,7 @@ static int launch_substep_3d(struct dgpu_ctx *c, int sub) {
   CK(cudaStreamWaitEvent(c->side2, c->fork[0], 0));
   CKK(dgk_merge(&c->d, sub, c->side));
   CKK(dgk_zmerge(&c->d, sub, c->side2));
+  CKK(dgk_ring_mean(&c->d, c->side2));
   CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
   CK(cudaEventRecord(c->fork[1], c->side));
   CK(cudaStreamWaitEvent(c->stream, c->fork[1], 0));
@@ -962,6 +974,7 @@ int dgpu_step_rk2_timed(dgpu_ctx *c, int nsteps, double *kernel_ms) {
       CKK(dgk_cellprep(&c->d, NULL, sub, c->stream));
       CK(cudaEventRecord(ev[e++], c->stream));
       CKK(dgk_merge(&c->d, sub, c->stream));
+      CKK(dgk_ring_mean(&c->d, c->stream));
       CKK(dgk_zmerge(&c->d, sub, c->stream));
       CK(cudaEventRecord(ev[e++], c->stream));
       CKK(dgk_rslope(&c->d, NULL, c->stream));
@@ -1095,6 +1108,7 @@ int dgpu_stage(dgpu_ctx *c, int phase) {
   }
   CKK(dgk_cellprep(&h, NULL, sub, c->stream));
   CKK(dgk_merge(&h, sub, c->stream));
+  CKK(dgk_ring_mean(&h, c->stream));
   /* the CFL minimum comes from k_plm_r (and dt from it, stored here for the
    * phases before k_update stores it); PLM results are kept only from phase 1 on */
   CKK(dgk_rslope(&h, NULL, c->stream));

@@ -169,6 +169,7 @@ typedef struct {
   double *fS;             /* [5][n_slots] r-face slopes (WR - WL)/(deltaR + deltaL) */
   double *fdp;            /* [2][n_slots] r-face offsets dpL, dpR (wrapped to [-pi, pi]) */
   double *ann_c;          /* [4][n_ann] per substep: kappa, cos(kappa dt), sin(kappa dt), 1-exp(-rate dt) */
+  int has_rigid;          /* some disk has w_numeric C_RIGID */
   const int *vz;          /* vz[0]: some disk may have a v_z (no_vz); NULL: taken as so */
   int form_dt;            /* substep 1 forms dt from dtkey where it is read (step_dt); 0: dgk_dt or
                              dgk_set_dt has stored it */
@@ -268,6 +269,8 @@ int dgk_merge(const DevPtrs *d, int substep, void *stream);
  * readers of InstState.dt) */
 int dgk_dt(const DevPtrs *d, void *stream);
 int dgk_source(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
+/* cell_set_w of the rigidly rotating disks (nothing without one) */
+int dgk_ring_mean(const DevPtrs *d, void *stream);
 int dgk_rslope(const DevPtrs *d, const TanPtrs *t, void *stream);
 int dgk_plm_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
 int dgk_flux_phi(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);

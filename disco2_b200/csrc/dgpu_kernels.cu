@@ -5,6 +5,8 @@
 //                                 / build_jloop) as a checked parallel merge of
 //                                 the two sorted phi-edge lists, cell_set_w
 //                                 and the frame terms of a moving frame
+//                                 (k_ring_mean per annulus: cell_set_w of a
+//                                 rigidly rotating mesh)
 //   k_cellprep per cell         : cell_clean_pi, cell_plm_p, GravMass copy /
 //                                 clean_pi
 //   k_rslope   per r face       : the face slope S and the wrapped offsets of
@@ -269,6 +271,65 @@ __device__ __forceinline__ void milos_frame(const DevPtrs &d, const DiskParams &
   d.frame[(size_t)lane * d.n_ann + a] = v;
 }
 
+// C_RIGID (cell_set_w.c:41-49): the mass-weighted mean v_phi of annulus a,
+// summed in j order like the reference, by one warp.  Its two sums are chains
+// of dependent additions (8.2 cycles each on B200), so all else is kept out of
+// them: the warp loads 128 cells ahead, puts the terms in shared memory, and
+// even lanes add those of one sum while odd lanes add the other's.  (With a
+// lane loading and adding cell by cell 32 us for 96 annuli of up to 660 cells;
+// with 32 cells ahead and the terms shuffled to every lane 24.)
+#define RING_CHUNK 128
+__device__ __forceinline__ void ring_mean(const DevPtrs &d, int a, int lane, double (&sh)[2][RING_CHUNK]) {
+  constexpr int K = RING_CHUNK / 32;
+  const unsigned full = 0xffffffffu;
+  const Annulus &A = d.ann[a];
+  const Pl QS = {d.qs};
+  const int np = A.np, off = A.cell_off;
+  const double r = A.r;
+  double u[K], m[K], sum = 0.0;
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const int c = off + min(j + 32 * i + lane, np - 1);
+      u[i] = ldr(d.prim, D_UPP, QS, c);
+      m[i] = ldr(d.cons, D_DDD, QS, c);
+    }
+  };
+  fetch(0);
+  for (int j = 0; j < np; j += RING_CHUNK) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      sh[0][32 * i + lane] = r * u[i] * m[i];
+      sh[1][32 * i + lane] = m[i];
+    }
+    __syncwarp();
+    if (j + RING_CHUNK < np) fetch(j + RING_CHUNK);
+    const double *t = sh[lane & 1];
+    if (np - j >= RING_CHUNK) {
+#pragma unroll 16
+      for (int k = 0; k < RING_CHUNK; ++k) sum += t[k];
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < np - j; ++k) sum += t[k];
+    }
+    __syncwarp();
+  }
+  const double w = __shfl_sync(full, sum, 0), Mring = __shfl_sync(full, sum, 1);
+  if (lane == 0) d.w_ann[a] = w / Mring;
+}
+
+// The ring means of the rigidly rotating disks, a warp per annulus, beside
+// k_merge and k_cellprep (only k_plm_r's CFL and later kernels read them; at
+// the end of the merge's blocks they stood in the step's chain: Gresho vortex,
+// 96 annuli, 0.105 -> 0.090 ms a step).
+#define RING_BLK 64
+__global__ void __launch_bounds__(RING_BLK) k_ring_mean(DevPtrs d) {
+  __shared__ double sh[RING_BLK / 32][2][RING_CHUNK];
+  const int a = (blockIdx.x * RING_BLK + threadIdx.x) / 32;
+  if (a < d.n_ann && d.par[d.ann[a].inst].w_numeric == DC_RIGID)
+    ring_mean(d, a, threadIdx.x & 31, sh[threadIdx.x / 32]);
+}
+
 // Per annulus pair (i, i+1) of a disk, one block: the r-face list of
 // face_create/build_jloop (src/Face/face_create_destroy.c:22-193) as a checked
 // parallel merge, and cell_set_w (src/Cell/cell_set_w.c:12-102) of annulus i.
@@ -288,9 +349,7 @@ __device__ __forceinline__ void merge_pair(const DevPtrs &d, int a, int substep)
   const double *traw = substep == 1 ? d.tiph0 : d.tiph1;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int np = A.np, off = A.cell_off;
-  const Pl QS = {d.qs};
-  const bool rigid = P.w_numeric == DC_RIGID;
-  if (!Z && tid == 0 && !rigid) d.w_ann[a] = A.wnum;
+  if (!Z && tid == 0 && P.w_numeric != DC_RIGID) d.w_ann[a] = A.wnum;
   if (!Z && tid >= nt - 32 && P.w_analytic == DA_MILOS) milos_frame(d, P, A, a, tid & 31);
   // the pair's arrays: r faces of (a, a+1), or z faces of (a, a+NR)
   int *const pfL = Z ? d.zfL : d.fL, *const pfR = Z ? d.zfR : d.fR;
@@ -504,44 +563,6 @@ __device__ __forceinline__ void merge_pair(const DevPtrs &d, int a, int substep)
       // slab slots past the list hold no face
       for (int n = nf + tid; n < c.cap; n += nt) c.fL[n] = -1;
     }
-  }
-  // C_RIGID: the mass-weighted mean v_phi of the annulus, summed in j order
-  // like the reference (cell_set_w.c:41-49), after the merge.  The sum is one
-  // chain of dependent additions, so what can be shortened is all else: the
-  // last warp loads 32 cells at a time (the next 32 while it adds these) and
-  // every lane adds the same shuffled terms in j order (Gresho vortex, 96
-  // annuli of up to 660 cells: this kernel 48 -> 29 us, the step 0.171 -> 0.133
-  // ms, against one lane loading and adding cell by cell).
-  if (!Z && rigid && tid >= nt - 32) {
-    const unsigned full = 0xffffffffu;
-    const int lane = tid & 31;
-    double w = 0.0, Mring = 0.0, x = 0.0, m = 0.0;
-    auto fetch = [&](int j, double &xj, double &mj) {
-      if (j >= np) return;
-      const double vp = A.r * ldr(d.prim, D_UPP, QS, off + j);
-      mj = ldr(d.cons, D_DDD, QS, off + j);
-      xj = vp * mj;
-    };
-    fetch(lane, x, m);
-    for (int j = 0; j < np; j += 32) {
-      double xn = 0.0, mn = 0.0;
-      fetch(j + 32 + lane, xn, mn);
-      if (np - j >= 32) {
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          Mring += __shfl_sync(full, m, k);
-          w += __shfl_sync(full, x, k);
-        }
-      } else {
-        for (int k = 0; k < np - j; ++k) {
-          Mring += __shfl_sync(full, m, k);
-          w += __shfl_sync(full, x, k);
-        }
-      }
-      x = xn;
-      m = mn;
-    }
-    if (lane == 0) d.w_ann[a] = w / Mring;
   }
 }
 
@@ -1537,13 +1558,14 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, T
 template <int MB>
 __global__ void __launch_bounds__(BLK, MB) k_prep(DevPtrs d, int substep) {
   __shared__ unsigned long long sh_k[BLK / 32];
-  __shared__ double sh_rk[6];
+  __shared__ double sh_rk[6], sh_ring[2][RING_CHUNK];
   const int a = blockIdx.x;
   const TanPtrs tp = {};
   merge_pair<false>(d, a, substep);
-  __syncthreads();  // w_ann[a] (one lane) before the CFL
   const Annulus &A = d.ann[a];
   const DiskParams &P = d.par[A.inst];
+  if (P.w_numeric == DC_RIGID && threadIdx.x >= BLK - 32) ring_mean(d, a, threadIdx.x & 31, sh_ring);
+  __syncthreads();  // w_ann[a] (one lane) before the CFL
   for (int j = threadIdx.x; j < A.np; j += BLK) cellprep_cell<double, false>(d, tp, A.cell_off + j, substep);
   if (threadIdx.x == 0) {
     d.sweep_flag[a] = 0;
@@ -2100,6 +2122,11 @@ int dgk_cellprep(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) 
 }
 int dgk_merge(const DevPtrs *d, int substep, void *stream) {
   k_merge<<<d->n_ann, d->merge_nt > 0 ? d->merge_nt : BLK, d->smem_face, (cudaStream_t)stream>>>(*d, substep);
+  return (int)cudaGetLastError();
+}
+int dgk_ring_mean(const DevPtrs *d, void *stream) {
+  if (!d->has_rigid) return 0;
+  k_ring_mean<<<(d->n_ann + RING_BLK / 32 - 1) / (RING_BLK / 32), RING_BLK, 0, (cudaStream_t)stream>>>(*d);
   return (int)cudaGetLastError();
 }
 int dgk_rslope(const DevPtrs *d, const TanPtrs *t, void *stream) {

@@ -2,8 +2,8 @@
 kernels change path, against the oracle's C restatement run on the host: the
 Gresho vortex reaches no transcendental, so the states are equal bit for bit.
 
-Ring means are added 32 cells at a time (rings of 31 to 65 cells); outflow
-boundary cells take 8 faces at a time, and a disk of three annuli chains all
+Ring means are added 128 cells at a time, loaded 32 by 32; outflow boundary
+cells take 8 faces at a time, and a disk of three annuli chains all
 three passes.
 """
 import os
@@ -16,7 +16,7 @@ from disco2_b200 import configs, lib
 
 pytestmark = pytest.mark.gpu
 
-RINGS = [{"NP_CONST": n} for n in (2, 31, 32, 33, 64, 65)]
+RINGS = [{"NP_CONST": n} for n in (2, 31, 32, 33, 65, 127, 128, 129, 257)]
 OUT = {"BoundTypeR": 1}
 OUTFLOW = [
     {"num_r": 1, "NP_CONST": 7, **OUT},                      # three annuli
