@@ -169,7 +169,6 @@ typedef struct {
   double *fS;             /* [5][n_slots] r-face slopes (WR - WL)/(deltaR + deltaL) */
   double *fdp;            /* [2][n_slots] r-face offsets dpL, dpR (wrapped to [-pi, pi]) */
   double *ann_c;          /* [4][n_ann] per substep: kappa, cos(kappa dt), sin(kappa dt), 1-exp(-rate dt) */
-  int has_rigid;          /* some disk has w_numeric C_RIGID */
   const int *vz;          /* vz[0]: some disk may have a v_z (no_vz); NULL: taken as so */
   int form_dt;            /* substep 1 forms dt from dtkey where it is read (step_dt); 0: dgk_dt or
                              dgk_set_dt has stored it */
@@ -202,6 +201,7 @@ typedef struct {
   /* z faces of 3-D disks (NZ > 1): the same structures as the r faces, per
      z pair (ring a, ring a+NR) of each ring a with k < NZ-1 */
   int n_zslots, n_zruns, has_z;
+  int has_rigid;          /* some disk has w_numeric C_RIGID */
   const int *zslot_ann;   /* z-face slot -> ring of its pair (the lower ring) */
   int *zfL, *zfR;         /* z-face cells (global); zfL = -1 past the list of a pair */
   double *zfdphi, *zfcm;

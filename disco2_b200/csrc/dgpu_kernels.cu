@@ -2164,8 +2164,20 @@ int dgk_source(const DevPtrs *d, const TanPtrs *t, int substep, void *stream) {
 }
 // k_update's blocks: the cells', and the GravMass block with tail > 0
 static int update_grid(const DevPtrs *d, int tail) { return (d->n_cells + TBLK - 1) / TBLK + (tail > 0); }
-int dgk_update(const DevPtrs *d, const TanPtrs *t, int substep, int stop, void *stream) {
+// k_update's resident blocks of BLK threads per SM where none was tuned: the
+// built-in 4 (64 registers, spills), or 3 (80) when the cells take as many
+// waves of the 148 SMs either way: 199,428 cells 30.7 -> 28.8 us (0.233 ->
+// 0.2275 ms a step), 59,746 cells 16.4 -> 15; with a wave more 258,078 cells
+// go from 35.5 to 39.
+static int update_blocks_per_sm(const DevPtrs *d) {
+  const long long c3 = 148LL * 3 * BLK, c4 = 148LL * 4 * BLK, n = d->n_cells;
+  return (n + c3 - 1) / c3 == (n + c4 - 1) / c4 ? 3 : DGPU_MINB_UPDATE;
+}
+int dgk_update(const DevPtrs *d0, const TanPtrs *t, int substep, int stop, void *stream) {
   int tail = stop >= 7 ? 2 : (stop >= 5 ? 1 : 0);
+  DevPtrs h = *d0;
+  const DevPtrs *d = &h;
+  if (!h.tune[DGPU_TUNE_UPDATE]) h.tune[DGPU_TUNE_UPDATE] = update_blocks_per_sm(d0);
   DGK_LAUNCH_TUNED(k_update, DGPU_TUNE_UPDATE, DGPU_MINB_UPDATE, update_grid(d, tail), TBLK, stream, substep, stop, tail,
                   
                    (double *)NULL, (const int *)NULL);
