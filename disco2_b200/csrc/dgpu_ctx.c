@@ -4,7 +4,7 @@
  * A context owns the device copy of one or more disks: the annulus-major
  * structure-of-arrays state, the per-annulus tables, the r-face slabs and the
  * per-disk GravMass/time state.  One RK2 step (timestep_rk2,
- * src/TimeStep/timestep_algorithm.c:11-41) is eight kernel launches, captured
+ * src/TimeStep/timestep_algorithm.c:11-41) is two substeps of eight kernels, captured
  * once into a CUDA graph and replayed; no host synchronisation happens inside
  * a step (dt, t and the GravMass orbit live on the device).
  */
@@ -492,7 +492,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
   }
   /* the fused substep covers the forward step of disks without passive
    * scalars, outflow radial boundary or sink; it is opt-in (dgpu_set_fused):
-   * on B200 the eight-kernel graph is faster (0.375 against 0.55 ms per step
+   * on B200 the eight-kernel graph is faster (0.284 against 0.51 ms per step
    * on the 258k-cell circumbinary disk) */
   c->fused_ok = c->n_pass == 0 && c->n_ob == 0 && !has_z;
   for (k = 0; k < n; ++k)

@@ -133,7 +133,8 @@ int dgpu_fused(const dgpu_ctx *ctx);
  * substep 2; for the fused one k_prep, k_sweep of substep 1 in [0], [1] and of
  * substep 2 in [8], [9].  Synchronous.  For measurement only: inside the step
  * graph of the eight kernels merge runs beside cellprep, and source and
- * flux_phi beside flux_r. */
+ * flux_phi beside flux_r (a rigid mesh's ring means are timed with the merge,
+ * the outflow boundary with the update). */
 int dgpu_step_rk2_timed(dgpu_ctx *ctx, int nsteps, double *kernel_ms);
 /* Autotuner (no counterpart in the reference): chooses how many blocks of 256
  * threads each SM should hold for the heavy step kernels (the register budget
