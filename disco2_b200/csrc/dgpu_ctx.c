@@ -422,7 +422,7 @@ int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dg
     c->d.pair_T = (int *)dmalloc(sizeof(int) * A, &ok);
     c->d.pair_seq = (int *)dmalloc(sizeof(int) * A, &ok);
     c->d.runs = (int *)dmalloc(sizeof(int) * (size_t)(c->n_runs ? c->n_runs : 1), &ok);
-    c->d.mdot_part = (double *)dmalloc(sizeof(double) * 2 * (size_t)c->n_upd_blocks, &ok);
+    c->d.mdot_part = (double *)dmalloc(sizeof(double) * 2 * ((size_t)c->n_upd_blocks + (size_t)n), &ok);
     c->d.counters = (unsigned int *)dmalloc(sizeof(unsigned int) * 8, &ok);
     c->d.cfl_ann = (unsigned long long *)dmalloc(sizeof(unsigned long long) * A, &ok);
     c->d.sweep_flag = (int *)dmalloc(sizeof(int) * A, &ok);

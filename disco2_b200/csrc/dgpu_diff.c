@@ -327,7 +327,7 @@ static int alloc_shadow(struct dgpu_ctx *c, DevPtrs *h, void **mem) {
   SZ(8 * 2 * S);               /* 11: fdphi fcm */
   SZ(4 * 4 * A);               /* 12: pair_nf pair_jpmin pair_T pair_seq */
   SZ(4 * R);                   /* 13: runs */
-  SZ(8 * 2 * B);               /* 14: mdot_part */
+  SZ(8 * 2 * (B + (size_t)c->n_inst)); /* 14: mdot_part */
   SZ(4 * 8);                   /* 15: counters */
   SZ(sizeof(InstState) * (size_t)c->n_inst); /* 16: ist */
   SZ(8 * DGPU_FR_N * A);       /* 17: frame */

@@ -183,7 +183,7 @@ typedef struct {
   double *fdphi, *fcm;    /* r-face dphi and cm */
   int *pair_nf, *pair_jpmin, *pair_T, *pair_seq; /* per annulus (pair i, i+1) */
   int *runs;              /* run starts */
-  double *mdot_part;      /* [n_blocks_update][2] per-block sink sums */
+  double *mdot_part;      /* [n_upd_blocks + n_inst][2] sink sums per block and disk (mdot_slot) */
   unsigned int *counters; /* last-block counters */
   int *err;               /* error flags */
   double *obuf;           /* [5 + n_pass][n_ob] prims, before damping, of the annuli the outflow

@@ -1329,9 +1329,15 @@ __device__ __forceinline__ void source_cell_k(const DevPtrs &d, const TanPtrs &t
   }
 }
 
+// The place in mdot_part of disk k's sink sums over the cells of block b: one
+// apart from block to block and from disk to disk, so no two of them share one
+// (at most n_inst more than there are blocks).
+__device__ __forceinline__ size_t mdot_slot(int b, int k) { return (size_t)b + (size_t)k; }
+
 template <typename T, int MB = DGPU_MINB_SOURCE, bool PS = false, bool V4 = forward_v4<T, PS>>
 __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int substep, int cells) {
   __shared__ double sh_md[2][BLK / 32];
+  __shared__ int sh_k[2];  // the first and the last cell's disk
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int N = d.n_cells;
   const double fac = substep == 1 ? 1.0 : 0.5;
@@ -1341,33 +1347,56 @@ __global__ void __launch_bounds__(BLK, MB) k_source(DevPtrs d, TanPtrs tp, int s
     ann_consts(d, t, S, fac * step_dt(d, S, d.par[inst], substep));
   }
   double md0 = 0.0, md1 = 0.0;
+  int inst = 0;
   if (t < N && cells) {
-    const int inst = d.ann[d.cell_ann[t]].inst;
+    inst = d.ann[d.cell_ann[t]].inst;
     const InstState &S = d.ist[inst];
     const double dt = fac * step_dt(d, S, d.par[inst], substep);
     if (V4 && no_vz(d)) source_cell_k<T, PS, V4 ? 4 : 5>(d, tp, t, S, dt, md0, md1);
     else source_cell_k<T, PS>(d, tp, t, S, dt, md0, md1);
   }
-  // deterministic per-block Mdot partial sums (reduced in block order by k_update)
-  const unsigned full = 0xffffffffu;
+  // deterministic Mdot partial sums, one per block and disk in it (mdot_slot;
+  // reduced in block order by k_update).  The sums over the whole block first,
+  // which are the disk's where the block holds one; else disk after disk.
+  auto partial = [&](double m0, double m1) {
+    const unsigned full = 0xffffffffu;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    md0 += __shfl_down_sync(full, md0, o);
-    md1 += __shfl_down_sync(full, md1, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    sh_md[0][threadIdx.x >> 5] = md0;
-    sh_md[1][threadIdx.x >> 5] = md1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && (size_t)blockIdx.x * BLK < (size_t)N) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int w = 0; w < BLK / 32; ++w) {
-      s0 += sh_md[0][w];
-      s1 += sh_md[1][w];
+    for (int o = 16; o > 0; o >>= 1) {
+      m0 += __shfl_down_sync(full, m0, o);
+      m1 += __shfl_down_sync(full, m1, o);
     }
-    d.mdot_part[2 * blockIdx.x] = s0;
-    d.mdot_part[2 * blockIdx.x + 1] = s1;
+    if ((threadIdx.x & 31) == 0) {
+      sh_md[0][threadIdx.x >> 5] = m0;
+      sh_md[1][threadIdx.x >> 5] = m1;
+    }
+    __syncthreads();
+  };
+  auto store = [&](int k) {
+    if (threadIdx.x == 0) {
+      double s0 = 0.0, s1 = 0.0;
+      for (int w = 0; w < BLK / 32; ++w) {
+        s0 += sh_md[0][w];
+        s1 += sh_md[1][w];
+      }
+      double *p = d.mdot_part + 2 * mdot_slot(blockIdx.x, k);
+      p[0] = s0;
+      p[1] = s1;
+    }
+  };
+  if ((size_t)blockIdx.x * BLK >= (size_t)N) return;
+  if (threadIdx.x == 0) sh_k[0] = inst;
+  if (t == min((int)(blockIdx.x + 1) * BLK, N) - 1) sh_k[1] = inst;
+  partial(md0, md1);
+  const int k0 = sh_k[0], k1 = sh_k[1];
+  if (k0 == k1) {
+    store(k0);
+    return;
+  }
+  for (int k = k0; k <= k1; ++k) {
+    __syncthreads();
+    const bool mine = t < N && inst == k;
+    partial(mine ? md0 : 0.0, mine ? md1 : 0.0);
+    store(k);
   }
 }
 
@@ -1524,14 +1553,14 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, T
       InstState &S = d.ist[k];
       const DiskParams &P = d.par[k];
       if (substep == 1 && d.form_dt) S.dt = cfl_dt(S, P);
-      // Mdot of this disk: block partials in block order
+      // Mdot of this disk: its partials in block order
       const int c0 = P.cell_base, c1 = P.cell_base + P.n_cells;
       const int b0 = c0 / BLK, b1 = (c1 + BLK - 1) / BLK;
       double s0 = 0.0, s1 = 0.0;
       if (P.rho_sink_on == 1) {
         for (int m = b0; m < b1; ++m) {
-          s0 += d.mdot_part[2 * m];
-          s1 += d.mdot_part[2 * m + 1];
+          s0 += d.mdot_part[2 * mdot_slot(m, k)];
+          s1 += d.mdot_part[2 * mdot_slot(m, k) + 1];
         }
       }
       S.mdot[0] = s0;
