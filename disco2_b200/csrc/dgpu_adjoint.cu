@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   for (int q = 0; q < 5; ++q) {
     double m = gq[q] / dAtot;
     if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      if (fabs(lim[q] * m) > 1.e-290 * plm) {
+      if (limit_decided(lim[q], m, plm)) {
         sel[q] = -2;
       } else {
         // an underflowing product or a zero slope: the forward's loop itself

@@ -608,6 +608,16 @@ HD void visc_flux(const ViscIn<T> &v, int dir, const DiskParams &P, const GravT<
   }
 }
 
+// Whether the one-walk limiter of the face slopes (plm_r_grad, k_plm_z,
+// a_gather_plm) may give 0 for a mean m that some face slope S opposes, as the
+// reference's face-by-face loop does.  The loop's running slope is m or some
+// plm * S, so at least the smaller of |m| and |lim| in size (lim: the plm * S
+// nearest zero), and the opposing S is at least |lim| / plm: where their
+// product cannot underflow, the loop sees the opposition.
+HD bool limit_decided(double lim, double m, double plm) {
+  return fabs(lim) * fmin(fabs(lim), fabs(m)) > 1.e-290 * plm;
+}
+
 // ---------------------------------------------------------------------------
 // Per-cell pieces of the substep shared by the forward, tangent and adjoint
 // ---------------------------------------------------------------------------

@@ -650,9 +650,10 @@ __device__ __noinline__ void limit_seq(const DevPtrs &d, const TanPtrs &tp, int 
 // needs: the plm * S nearest zero (the first of equals) and whether any S was
 // negative or positive.  The limiter then gives 0 if some S opposes the mean,
 // else the nearer of the mean and that plm * S, which is where the reference's
-// face-by-face loop ends.  It would not where a product S * mean of opposed
-// signs underflows to -0 (or an S is 0), so that its test S * mean < 0 fails:
-// those planes run the loop itself (limit_seq).  Two walks, one for the sum and
+// face-by-face loop ends.  It would not where the product of an opposing S and
+// the loop's running slope, which an earlier face may have clipped, underflows
+// to -0 (or an S is 0), so that its test S * slope < 0 fails: planes where that
+// could be (limit_decided) run the loop itself (limit_seq).  Two walks, one for the sum and
 // one for the limiter, took 229 us in substep 2 of 16 disks (4 M cells) and
 // 23.5 us of one 258,078-cell disk against 191 and 19.3 here.  Forming each S
 // here from the cell across the face, with no slopes stored, took 495 us for
@@ -705,8 +706,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
   for (int q = 0; q < NV; ++q) {
     T m = gq[q] / dAtot;
     if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      // every product S * m is at least |lim| |m| / plm in size
-      if (fabs(val(lim[q]) * val(m)) > 1.e-290 * plm) m = 0.0;
+      if (limit_decided(val(lim[q]), val(m), plm)) m = 0.0;
       else seq |= 1 << q;
     } else if (fabs(lim[q]) < fabs(m)) {
       m = lim[q];
@@ -1105,8 +1105,7 @@ __global__ void __launch_bounds__(BLK) k_plm_z(const __grid_constant__ DevPtrs d
   for (int q = 0; q < 5; ++q) {
     double m = gq[q] / dAtot;
     if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      // every product S * m is at least |lim| |m| / plm in size
-      if (fabs(lim[q] * m) > 1.e-290 * plm) m = 0.0;
+      if (limit_decided(lim[q], m, plm)) m = 0.0;
       else seq |= 1 << q;
     } else if (fabs(lim[q]) < fabs(m)) {
       m = lim[q];
