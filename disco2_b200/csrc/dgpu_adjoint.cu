@@ -635,14 +635,15 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   // the same walk keeps what the limiter of the forward needs (plm_r_grad):
   // the mean's sum, the plm * S nearest zero and its face, and the signs seen
   double gq[5], lim[5];
-  int sel[5], neg = 0, pos = 0;  // sel: the clipping slot; then -1 the average, -2 zero
+  const double plm = P.plm;
+  int sel[5];  // the clipping slot; then -1 the average, -2 zero
+  int neg = plm < 0.0 ? 31 : 0, pos = neg;  // (a negative PLM: always the loop)
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     gq[q] = 0.0;
     lim[q] = HUGE_VAL;
     sel[q] = -1;
   }
-  const double plm = P.plm;
   for_cell_rfaces(d, A, a, g, P.NR, [&](const RFace &F, int slot, int asR) {
     const double *src = asR ? J.arR : J.arL;
 #pragma unroll
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(BLK) a_gather_plm(DevPtrs d, AdjPtrs J) {
   for (int q = 0; q < 5; ++q) {
     double m = gq[q] / dAtot;
     if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      if (limit_decided(lim[q], m, plm)) {
+      if (fabs(lim[q] * (fabs(lim[q]) < fabs(m) ? lim[q] : m)) > limit_floor(plm)) {
         sel[q] = -2;
       } else {
         // an underflowing product or a zero slope: the forward's loop itself

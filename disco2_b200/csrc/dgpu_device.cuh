@@ -608,14 +608,27 @@ HD void visc_flux(const ViscIn<T> &v, int dir, const DiskParams &P, const GravT<
   }
 }
 
-// Whether the one-walk limiter of the face slopes (plm_r_grad, k_plm_z,
-// a_gather_plm) may give 0 for a mean m that some face slope S opposes, as the
-// reference's face-by-face loop does.  The loop's running slope is m or some
-// plm * S, so at least the smaller of |m| and |lim| in size (lim: the plm * S
-// nearest zero), and the opposing S is at least |lim| / plm: where their
-// product cannot underflow, the loop sees the opposition.
-HD bool limit_decided(double lim, double m, double plm) {
-  return fabs(lim) * fmin(fabs(lim), fabs(m)) > 1.e-290 * plm;
+// The end of the one-walk limiter of the face slopes (plm_r_grad, k_plm_z and,
+// by branch, a_gather_plm): from the mean m and lim, the plm * S nearest zero,
+// the slope at which the reference's face-by-face loop ends.  opposed: some
+// face slope S has the sign that m has not.  Without one the loop ends at the
+// nearer of m and lim.  With one it ends at 0, unless the product of S and the
+// running slope underflows: that slope is m or some plm * S, so at least the
+// smaller of |m| and |lim| in size, and the opposing S is at least |lim| / plm.
+// Returns true where that could be (m is left as it is, for the loop itself).
+// floor: limit_floor(plm).  A negative PLM turns the running slope's sign at
+// every clip, which only the loop follows: opposed has to be true for it.
+HD double limit_floor(double plm) { return plm < 0.0 ? HUGE_VAL : 1.e-290 * plm; }
+template <typename T>
+HD bool limit_left(T &m, const T &lim, bool opposed, double floor) {
+  const T w = fabs(lim) < fabs(m) ? lim : m;
+  if (!opposed) {
+    m = w;
+    return false;
+  }
+  if (!(fabs(val(lim) * val(w)) > floor)) return true;
+  m = 0.0;
+  return false;
 }
 
 // ---------------------------------------------------------------------------

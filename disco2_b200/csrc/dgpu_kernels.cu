@@ -653,7 +653,7 @@ __device__ __noinline__ void limit_seq(const DevPtrs &d, const TanPtrs &tp, int 
 // face-by-face loop ends.  It would not where the product of an opposing S and
 // the loop's running slope, which an earlier face may have clipped, underflows
 // to -0 (or an S is 0), so that its test S * slope < 0 fails: planes where that
-// could be (limit_decided) run the loop itself (limit_seq).  Two walks, one for the sum and
+// could be (limit_left) run the loop itself (limit_seq).  Two walks, one for the sum and
 // one for the limiter, took 229 us in substep 2 of 16 disks (4 M cells) and
 // 23.5 us of one 258,078-cell disk against 191 and 19.3 here.  Forming each S
 // here from the cell across the face, with no slopes stored, took 495 us for
@@ -670,7 +670,7 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
   const DiskParams &P = d.par[A.inst];
   const double plm = P.plm;
   T gq[5], lim[5];
-  int neg = 0, pos = 0;
+  int neg = plm < 0.0 ? 31 : 0, pos = neg;  // (a negative PLM: always the loop)
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
     gq[q] = 0.0;
@@ -701,16 +701,13 @@ __device__ __forceinline__ void plm_r_grad(const DevPtrs &d, const TanPtrs &tp, 
     else if (A.i == P.NR - 1) dAtot = dz * A.rm * dp;
     else dAtot = dz * (A.rp + A.rm) * dp;
   }
+  const double floor = limit_floor(plm);
   int seq = 0;  // planes that run the loop itself
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
     T m = gq[q] / dAtot;
-    if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      if (limit_decided(val(lim[q]), val(m), plm)) m = 0.0;
-      else seq |= 1 << q;
-    } else if (fabs(lim[q]) < fabs(m)) {
-      m = lim[q];
-    }
+    const bool opposed = (m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1));
+    seq |= limit_left(m, lim[q], opposed, floor) << q;
     gq[q] = m;
   }
   stk<NV, T>(d.grad, tp.grad, 0, QS, g, gq);
@@ -1077,7 +1074,7 @@ __global__ void __launch_bounds__(BLK) k_plm_z(const __grid_constant__ DevPtrs d
   const double rm = A.rm, rp = A.rp, plm = P.plm;
   const double zr = .5 * (rp + rm), zperp = rp - rm;  // build_jloop's r and deltaPerp of a z face
   double gq[5], lim[5];
-  int neg = 0, pos = 0;
+  int neg = plm < 0.0 ? 31 : 0, pos = neg;  // (a negative PLM: always the loop)
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     gq[q] = 0.0;
@@ -1100,16 +1097,13 @@ __global__ void __launch_bounds__(BLK) k_plm_z(const __grid_constant__ DevPtrs d
   });
   const double dp = d.dphi[g];
   const double dAtot = 2. * .5 * (rp * rp - rm * rm) * dp;
+  const double floor = limit_floor(plm);
   int seq = 0;  // planes that run the loop itself
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     double m = gq[q] / dAtot;
-    if ((m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1))) {
-      if (limit_decided(lim[q], m, plm)) m = 0.0;
-      else seq |= 1 << q;
-    } else if (fabs(lim[q]) < fabs(m)) {
-      m = lim[q];
-    }
+    const bool opposed = (m < 0.0 && (pos >> q & 1)) || (m > 0.0 && (neg >> q & 1));
+    seq |= limit_left(m, lim[q], opposed, floor) << q;
     gq[q] = m;
   }
   stk<5>(d.gradz, 0, P5, g, gq);

@@ -27,12 +27,12 @@ static double loop(const double *S, int n, double m, double plm) {
 
 int main() {
   const int ex[] = {-310, -300, -200, -170, -160, -150, -145, -140, -100, -17, 0, 100};
-  const double plms[] = {1.0, 1.5, 2.0, 1e-3, 0.0};
+  const double plms[] = {1.0, 1.5, 2.0, 1e-3, 0.0, -0.7};
   long decided = 0, left = 0, wrong = 0;
   for (int t = 0; t < 4000000; ++t) {
     double S[5], m = 0.0;
     const int n = 2 + urand(4);
-    const double plm = plms[urand(5)];
+    const double plm = plms[urand(6)];
     const int lo = urand(12), hi = urand(12);
     for (int k = 0; k < n; ++k) {
       S[k] = urand(16) == 0 ? 0.0 : (1 + urand(9)) * pow(10.0, ex[urand(2) ? lo : hi]);
@@ -42,7 +42,7 @@ int main() {
     m /= n;
     // the kernels' walk
     double lim = HUGE_VAL;
-    bool neg = false, pos = false;
+    bool neg = plm < 0.0, pos = neg;
     for (int k = 0; k < n; ++k) {
       const double ps = plm * S[k];
       if (fabs(ps) < fabs(lim)) lim = ps;
@@ -50,14 +50,10 @@ int main() {
       pos |= S[k] > 0.0;
     }
     double got = m;
-    if ((m < 0.0 && pos) || (m > 0.0 && neg)) {
-      if (!limit_decided(lim, m, plm)) {
-        ++left;
-        continue;
-      }
-      got = 0.0;
-    } else if (fabs(lim) < fabs(m)) {
-      got = lim;
+    if (limit_left(got, lim, (m < 0.0 && pos) || (m > 0.0 && neg), limit_floor(plm))) {
+      ++left;
+      if (got != m) ++wrong;
+      continue;
     }
     ++decided;
     if (got != loop(S, n, m, plm)) ++wrong;

@@ -62,3 +62,18 @@ def test_reverse_of_mixed_slopes():
     along = float((g["dprim"] * d).sum())
     scale = float(np.abs(g["dprim"] * d).sum())
     assert abs(along - dJ[1]) <= 1e-9 * scale
+
+
+def test_limiter_with_negative_plm(tmp_path):
+    """A PLM below zero turns the slope's sign at every face that clips it."""
+    p = configs.gresho(8, R_Min=0.2, PLM=-0.7)
+    par = configs.write_parfile(p, os.path.join(str(tmp_path), "g.par"))
+    st, _, _ = oracle.run(par, 0, impl="port")
+    st.prim += 0.05 * np.random.default_rng(1).uniform(-1.0, 1.0, st.prim.shape)
+    want = oracle.stage(par, 1, impl="port", load=st)
+    ctx = lib.Context(lib.Sim(p))
+    ctx.init_state(0)
+    ctx.set_state(0, st.prim, st.tiph, st.dphi)
+    ctx.stage(1)
+    assert np.array_equal(ctx.stage_data(0)["grad"], want.ext["grad"])
+    ctx.close()

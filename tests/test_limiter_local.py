@@ -1,5 +1,5 @@
 """The rule by which the one walk over a cell's face slopes decides the limiter
-(limit_decided: k_plm_r, k_plm_z and the reverse step's a_gather_plm) against
+(limit_left: k_plm_r, k_plm_z and, by branch, the reverse step's a_gather_plm) against
 the reference's face-by-face loop, on the host: slopes of mixed sizes, whose
 products with the running slope underflow in one order and not in another."""
 import os
