@@ -674,19 +674,19 @@ int dgpu_get_stage_data(dgpu_ctx *c, int inst, double *grad, double *gradp, doub
   }
   if (rktiph) CK(cudaMemcpyAsync(rktiph, c->d.rktiph + base, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
   if (wiph) {
-    /* wiph is one value per annulus */
-    const struct dgpu_sim *s = c->sims[inst];
-    double *w = (double *)malloc(sizeof(double) * (size_t)s->NR);
+    /* wiph is one value per annulus of every layer */
+    const int nrings = c->sims[inst]->NR * c->sims[inst]->NZ;
+    double *w = (double *)malloc(sizeof(double) * (size_t)nrings);
     int i, j, m = 0;
     if (!w) return fail(c, DGPU_ERR_NOMEM, "out of host memory");
-    if (cudaMemcpyAsync(w, c->d.w_ann + p->ann_base, sizeof(double) * (size_t)s->NR, cudaMemcpyDeviceToHost,
+    if (cudaMemcpyAsync(w, c->d.w_ann + p->ann_base, sizeof(double) * (size_t)nrings, cudaMemcpyDeviceToHost,
                         c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
       free(w);
       return fail(c, DGPU_ERR_CUDA, "wiph download failed");
     }
-    for (i = 0; i < s->NR; ++i)
-      for (j = 0; j < s->N_p[i]; ++j) wiph[m++] = w[i];
+    for (i = 0; i < nrings; ++i)
+      for (j = 0; j < c->h_ann[p->ann_base + i].np; ++j) wiph[m++] = w[i];
     free(w);
   }
   return dgpu_synchronize(c);
