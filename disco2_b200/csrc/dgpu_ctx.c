@@ -664,6 +664,7 @@ int dgpu_get_stage_data(dgpu_ctx *c, int inst, double *grad, double *gradp, doub
     double *srcs[3] = {c->d.grad, c->d.gradp, c->d.rkcons};
     double *dsts[3] = {grad, gradp, rkcons};
     int k;
+    if (grad || gradp || rkcons) CKK(dgk_clear_vz(&c->d, c->stream));
     for (k = 0; k < 3; ++k) {
       if (!dsts[k]) continue;
       CKK(dgk_soa_to_aos(c->d_stage, 5 + p->num_n, c->d.qs, base, srcs[k], n, c->stream));
@@ -1120,6 +1121,7 @@ int dgpu_stage(dgpu_ctx *c, int phase) {
     CKK(dgk_flux_r(&h, NULL, sub, c->stream));
   }
   CKK(dgk_update_stage(&h, sub, stop, c->stream));
+  CK(cudaMemsetAsync(c->d.counters + DGPU_CT_NO_VZ, 0, sizeof(unsigned int), c->stream));
   if (stop >= 6 && c->n_ob > 0) CKK(dgk_outflow(&h, stop, c->stream));
   /* from phase 5 of substep 1 on the advanced phi edges live in the substep's
    * output buffer (substep 2 writes them where the state is read) */

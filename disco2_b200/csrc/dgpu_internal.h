@@ -147,6 +147,8 @@ typedef struct {
 #define DGPU_FR_FRDROM 3 /* sim_rdrOm_a at the radius of the r-face pair */
 #define DGPU_FR_N 4
 
+#define DGPU_CT_NO_VZ 1
+
 /* Device pointers and sizes handed to every kernel. */
 typedef struct {
   int n_inst, n_ann, n_cells, n_slots, n_runs;
@@ -184,7 +186,7 @@ typedef struct {
   int *pair_nf, *pair_jpmin, *pair_T, *pair_seq; /* per annulus (pair i, i+1) */
   int *runs;              /* run starts */
   double *mdot_part;      /* [n_upd_blocks + n_inst][2] sink sums per block and disk (mdot_slot) */
-  unsigned int *counters; /* last-block counters */
+  unsigned int *counters; /* last-block counters; [DGPU_CT_NO_VZ]: the last substep left the v_z planes out */
   int *err;               /* error flags */
   double *obuf;           /* [5 + n_pass][n_ob] prims, before damping, of the annuli the outflow
                              boundary reads or writes (k_update writes them, k_outflow finishes them) */
@@ -323,6 +325,9 @@ int dgk_update_blocks(int n_cells);
 int dgk_block_size(void);
 int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos, int n, int *vz, void *stream);
 int dgk_any_vz(int *vz, int n_inst, void *stream);
+/* the v_z planes of grad, gradp and rkcons where the last substep left them
+ * out: the zeros it would have written */
+int dgk_clear_vz(const DevPtrs *d, void *stream);
 int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream);
 #ifdef __cplusplus
 }

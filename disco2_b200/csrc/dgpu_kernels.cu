@@ -1542,6 +1542,7 @@ __global__ void __launch_bounds__(TBLK, MB * (BLK / TBLK)) k_update(DevPtrs d, T
                                                                   int tail, double *rec, const int *rec_idx) {
   int b = blockIdx.x;
   if (tail > 0 && b-- == 0) {
+    if (threadIdx.x == 0) d.counters[DGPU_CT_NO_VZ] = V4 && no_vz(d);
     for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
       InstState &S = d.ist[k];
       const DiskParams &P = d.par[k];
@@ -1594,6 +1595,7 @@ __global__ void __launch_bounds__(BLK, MB) k_prep(DevPtrs d, int substep) {
     if (a == 0) {
       d.counters[3] = 0;
       d.counters[4] = 0;
+      d.counters[DGPU_CT_NO_VZ] = 0;
     }
   }
   if (substep != 1) return;
@@ -2069,6 +2071,13 @@ __global__ void k_any_vz(int *vz, int n_inst) {
   __syncthreads();
   if (threadIdx.x == 0) vz[0] = any;
 }
+__global__ void __launch_bounds__(BLK) k_clear_vz(DevPtrs d) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= d.n_cells || d.counters[DGPU_CT_NO_VZ] == 0) return;
+  const Pl QS = {d.qs};
+  d.grad[ix(D_UZZ, QS, g)] = d.gradp[ix(D_UZZ, QS, g)] = 0.0;
+  d.rkcons[ix(D_SZZ, QS, g)] = 0.0;
+}
 __global__ void k_soa_to_aos(double *aos, int nq, Pl planes, int base, const double *soa, int n) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -2086,6 +2095,10 @@ int dgk_aos_to_soa(double *soa, int nq, int planes, int base, const double *aos,
 }
 int dgk_any_vz(int *vz, int n_inst, void *stream) {
   k_any_vz<<<1, BLK, 0, (cudaStream_t)stream>>>(vz, n_inst);
+  return (int)cudaGetLastError();
+}
+int dgk_clear_vz(const DevPtrs *d, void *stream) {
+  k_clear_vz<<<(d->n_cells + BLK - 1) / BLK, BLK, 0, (cudaStream_t)stream>>>(*d);
   return (int)cudaGetLastError();
 }
 int dgk_soa_to_aos(double *aos, int nq, int planes, int base, const double *soa, int n, void *stream) {
