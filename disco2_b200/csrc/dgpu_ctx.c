@@ -1150,8 +1150,12 @@ static int face_list_dir(dgpu_ctx *c, int inst, int z, int cap, int *off, int *L
   nrings = s->NR * s->NZ;
   nslots = z ? c->d.n_zslots : c->n_slots;
   /* build the list of the current state: one merge pass (substep-1 buffers) */
-  if (z) CKK(dgk_zmerge(&c->d, 1, c->stream));
-  else CKK(dgk_merge(&c->d, 1, c->stream));
+  if (z) {
+    CKK(dgk_zmerge(&c->d, 1, c->stream));
+  } else {
+    CKK(dgk_merge(&c->d, 1, c->stream));
+    CKK(dgk_ring_mean(&c->d, c->stream)); /* (the merge sets the other meshes' w) */
+  }
   if ((rc = dgpu_synchronize(c))) return rc;
   nf = (int *)malloc(sizeof(int) * (size_t)nrings);
   fL = (int *)malloc(sizeof(int) * (size_t)(nslots > 0 ? nslots : 1));

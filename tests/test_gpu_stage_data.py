@@ -74,3 +74,23 @@ def test_stage_after_steps_without_vz():
         ctx.close()
     for k in KEYS:
         assert np.any(out[0][k][:, 4] != 0.0) and np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("make", [configs.gresho, configs.kepler_ring], ids=lambda f: f.__name__)
+def test_wiph_after_face_list(make):
+    """The face list of a newly set state brings wiph with it, on a rigidly
+    rotating mesh too (the ring means of that state)."""
+    sim = lib.Sim(make(9))
+    st = sim.initial_state()
+    prim = st["prim"].copy()
+    prim[:, 3] *= 1.5
+    ctx = lib.Context(sim)
+    ctx.init_state(0)
+    ctx.step(1)
+    ctx.set_state(0, prim, st["tiph"], st["dphi"])
+    ctx.face_list(0)
+    got = ctx.stage_data(0)["wiph"]
+    ctx.stage(0)
+    want = ctx.stage_data(0)["wiph"]
+    ctx.close()
+    assert np.array_equal(got, want)
