@@ -901,25 +901,29 @@ int dctx_launch_step(struct dgpu_ctx *c) {
   return DGPU_OK;
 }
 
+/* One RK2 step under the context's present launch shapes as a graph. */
+static int step_graph(struct dgpu_ctx *c, cudaGraphExec_t *out) {
+  cudaGraph_t g;
+  cudaError_t e;
+  int rc;
+  CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  rc = dctx_launch_step(c);
+  e = cudaStreamEndCapture(c->stream, &g);
+  if (rc) return rc;
+  if (e != cudaSuccess) return fail(c, DGPU_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return fail(c, DGPU_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
+  return DGPU_OK;
+}
+
 int dgpu_step_rk2(dgpu_ctx *c, int nsteps) {
   int k;
   if (!c || nsteps < 0) return DGPU_ERR_ARG;
   cudaSetDevice(c->device);
   if (!c->have_graph) {
-    cudaGraph_t g;
-    int rc;
-    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = dctx_launch_step(c);
-    {
-      cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-      if (rc) return rc;
-      if (e != cudaSuccess) return fail(c, DGPU_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-    }
-    {
-      cudaError_t e = cudaGraphInstantiate(&c->graph, g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return fail(c, DGPU_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
-    }
+    int rc = step_graph(c, &c->graph);
+    if (rc) return rc;
     c->have_graph = 1;
   }
   for (k = 0; k < nsteps; ++k) CK(cudaGraphLaunch(c->graph, c->stream));
@@ -1012,7 +1016,8 @@ int dgpu_step_rk2_timed(dgpu_ctx *c, int nsteps, double *kernel_ms) {
 
 /* The autotuner: a coordinate search over the resident blocks per SM of the
  * five heavy kernels (the register budget the compiler gets), each timed on
- * the context's own disks by dgpu_step_rk2_timed from the same saved state.
+ * the context's own disks by dgpu_step_rk2_timed from the same saved state,
+ * then the whole step under the result against the shapes there were.
  * The instances differ only in register allocation, so the results are
  * bitwise the same whatever is chosen. */
 #define TUNE_NCAND 4
@@ -1020,10 +1025,49 @@ static const int tune_cand[TUNE_NCAND] = {2, 3, 4, 5};
 /* kernel_ms slot of each tuned kernel in substep 1 (substep 2 is +8) */
 static const int tune_slot[DGPU_TUNE_N] = {3, 5, 6, 4, 7, 1};
 
+/* Whether the whole step is faster under the shapes b than under a, by more
+ * than the runs of either differ: TUNE_RUNS of `steps` steps each, in turn and
+ * from the saved state, b's slowest against a's fastest with 1% between them.
+ * A kernel that is faster alone need not be so beside the others: the shapes
+ * picked one by one made a step of 59,746 cells 103-105 us for the built-in
+ * 94.4, and one of 16 disks 3.70-3.82 ms for 3.65. */
+#define TUNE_RUNS 5
+static int tune_better(struct dgpu_ctx *c, const int *a, const int *b, int steps, double *buf, InstState *ist,
+                       int *better) {
+  cudaGraphExec_t g[2] = {NULL, NULL};
+  cudaEvent_t ev[2] = {NULL, NULL};
+  float best_a = 1e30f, worst_b = 0.f;
+  int k, r, s, rc = DGPU_OK;
+  for (k = 0; k < 2 && rc == DGPU_OK; ++k) {
+    memcpy(c->d.tune, k ? b : a, sizeof(c->d.tune));
+    rc = step_graph(c, &g[k]);
+    if (rc == DGPU_OK && cudaEventCreate(&ev[k]) != cudaSuccess)
+      rc = fail(c, DGPU_ERR_CUDA, "autotune: event creation failed");
+  }
+  for (r = 0; r < TUNE_RUNS && rc == DGPU_OK; ++r)
+    for (k = 0; k < 2 && rc == DGPU_OK; ++k) {
+      float ms = 0.f;
+      int bad = dgk_snap(&c->d, buf, ist, 0, c->stream) || cudaGraphLaunch(g[k], c->stream) ||
+                cudaEventRecord(ev[0], c->stream);
+      for (s = 0; s < steps && !bad; ++s) bad = cudaGraphLaunch(g[k], c->stream) != cudaSuccess;
+      if (bad || cudaEventRecord(ev[1], c->stream) || cudaEventSynchronize(ev[1]) ||
+          cudaEventElapsedTime(&ms, ev[0], ev[1]))
+        rc = fail(c, DGPU_ERR_CUDA, "autotune: timing the step failed");
+      else if (k == 0 && ms < best_a) best_a = ms;
+      else if (k == 1 && ms > worst_b) worst_b = ms;
+    }
+  for (k = 0; k < 2; ++k) {
+    if (g[k]) cudaGraphExecDestroy(g[k]);
+    if (ev[k]) cudaEventDestroy(ev[k]);
+  }
+  *better = rc == DGPU_OK && 1.01f * worst_b < best_a;
+  return rc;
+}
+
 int dgpu_autotune(dgpu_ctx *c, int steps, int *choice) {
   double *buf = NULL, ms[DGPU_STEP_KERNELS];
   InstState *ist = NULL;
-  int k, v, rc = DGPU_OK;
+  int k, v, rc = DGPU_OK, entry[DGPU_TUNE_N];
   static const int order[DGPU_TUNE_N - 1] = {DGPU_TUNE_UPDATE, DGPU_TUNE_FLUXR, DGPU_TUNE_FLUXPHI, DGPU_TUNE_SOURCE,
                                              DGPU_TUNE_PLM};
   static const int order_fused[1] = {DGPU_TUNE_SWEEP};
@@ -1045,6 +1089,7 @@ int dgpu_autotune(dgpu_ctx *c, int steps, int *choice) {
       cudaGetLastError();
       return fail(c, DGPU_ERR_NOMEM, "autotune: device allocation failed");
     }
+    memcpy(entry, c->d.tune, sizeof(entry));
     if (dgk_snap(&c->d, buf, ist, 1, c->stream)) rc = fail(c, DGPU_ERR_CUDA, "autotune: state save failed");
     /* the fused step tunes k_sweep (2..4 blocks per SM), the other the five
      * heavy kernels */
@@ -1073,6 +1118,13 @@ int dgpu_autotune(dgpu_ctx *c, int steps, int *choice) {
       }
       c->d.tune[kk] = bestv;
     }
+    if (rc == DGPU_OK && !c->fused && memcmp(entry, c->d.tune, sizeof(entry))) {
+      int tuned[DGPU_TUNE_N], better;
+      memcpy(tuned, c->d.tune, sizeof(tuned));
+      rc = tune_better(c, entry, tuned, steps, buf, ist, &better);
+      memcpy(c->d.tune, better ? tuned : entry, sizeof(entry));
+    }
+    if (rc) memcpy(c->d.tune, entry, sizeof(entry));
     if (rc == DGPU_OK && dgk_snap(&c->d, buf, ist, 0, c->stream))
       rc = fail(c, DGPU_ERR_CUDA, "autotune: state restore failed");
     if (rc == DGPU_OK) rc = dgpu_synchronize(c);

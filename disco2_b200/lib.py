@@ -328,8 +328,9 @@ class Context:
 
     def autotune(self, steps: int = 3, choice=None) -> dict:
         """Time each launch shape of the heavy kernels on this context's disks
-        and keep the fastest (steps == 0: apply `choice`); returns the blocks
-        per SM chosen for each tuned kernel."""
+        and keep the fastest if the whole step is faster with them (steps == 0:
+        apply `choice`); returns the blocks per SM chosen for each tuned kernel
+        (0: built-in)."""
         ch = (C.c_int * 6)(*(list(choice) + [0] * (6 - len(choice)) if choice is not None else [0] * 6))
         self._ck(load().dgpu_autotune(self._h, steps, ch))
         return dict(zip(self.TUNED, list(ch)))

@@ -142,7 +142,9 @@ int dgpu_step_rk2_timed(dgpu_ctx *ctx, int nsteps, double *kernel_ms);
  * current state with dgpu_step_rk2_timed (1 warm-up + `steps` steps per
  * choice), one kernel after the other: for the eight-kernel substep plm_r,
  * flux_phi, flux_r, source and update (2..5 each), for the fused one k_sweep
- * (2..4).  The state, t and the GravMass are restored afterwards, and results
+ * (2..4).  The eight-kernel substep's choice is kept only if the whole step is
+ * then faster than under the shapes the context had, by more than the runs
+ * differ.  The state, t and the GravMass are restored afterwards, and results
  * are bitwise the same under every choice.  choice[6] (may be NULL) receives
  * the chosen values in the order plm_r, flux_phi, flux_r, source, update,
  * sweep; with steps == 0 the given choice[6] is applied instead (0 = the
