@@ -302,8 +302,12 @@ HD void visc_flux_rev(const ViscIn<double> &v, int dir, const DiskParams &P, con
     x = r * cc;
     y = r * sc;
     // nu = alpha P / rho / sqrt(Q0 M0 + Q1 M1) with Q = (d^2 + eps^2)^-1.5 from
-    // reciprocal square roots, and no distance d (the forward's roundings need
-    // not be repeated here: 4.5 ulp at most, rms 0.77, against its 5.5 and 0.88)
+    // reciprocal square roots, and no distance d: the forward's roundings need
+    // not be repeated here.  The factor of nu against 80-bit arithmetic: 4.5 ulp
+    // at most, rms 0.77, where the quotients and roots have 5.5 and 0.88; the
+    // adjoints of the flux, medians over 200,000 faces (r 0.4-30, q 0.01-1), in
+    // units of 2^-53: binary positions 2.45-3.56 (2.52-3.90), masses 2.35-3.22
+    // (2.37-3.32), alpha 1.85 (1.87), cells 1.34-1.80 (1.36-1.81)
     const double eps = P.g_eps;
     s0 = (x - G.gx[0]) * (x - G.gx[0]) + (y - G.gy[0]) * (y - G.gy[0]) + eps * eps;
     s1 = (x - G.gx[1]) * (x - G.gx[1]) + (y - G.gy[1]) * (y - G.gy[1]) + eps * eps;
@@ -405,6 +409,10 @@ HD void source_cell_rev(const SrcGeom &g, const DiskParams &P, const double *pm,
   double Fr = 0.0, Fp = 0.0;
   double dx[2], dy[2], sr[2], cosa[2], sina[2], cosap[2], sinap[2], f1[2], sx[2], Qx[2];
   // for n = 2 the distance cancels: the force is -M (dx, dy) (d^2 + eps^2)^-1.5
+  // (adjoints of the source against 80-bit arithmetic, medians over 200,000
+  // cells in units of 2^-53, and with quotients and roots: binary positions
+  // 2.52-2.56 and 2.78-2.84, masses 2.30-2.41 and 2.43-2.55, density 4.54 and
+  // 4.82, the velocities 1.51-3.14 and 1.56-3.27)
   const bool n2 = P.phi_order == 2;
   for (int p = 0; p < 2; ++p) {
     dx[p] = g.gravdist * g.cosp - G.gx[p];

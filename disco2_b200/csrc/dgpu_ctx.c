@@ -241,7 +241,13 @@ void dgpu_destroy(dgpu_ctx *c) {
 }
 
 /* A context whose cell kernels run in at most two waves of blocks (148 SMs x
- * 4 blocks x 256 cells): its launches are bound by latency. */
+ * 4 blocks x 256 cells): its launches are bound by latency.  It forms dt where
+ * it is read (step_dt) and runs the phi faces on their own stream
+ * (dctx_substep).  Both against neither, us a step: 258,078 cells 280-288 and
+ * 291, 298,074 313-324 and 322-332; across the line the two differ little,
+ * 340,950 367-376 and 376, 469,908 502 and 511, 659,328 686-691 and 692-698,
+ * 1,029,762 1,043-1,070 and 1,048-1,054, and from 3 M cells neither is the
+ * faster (4.85 ms, 4.90 with the stream; 4.45, 4.48 with dt formed). */
 static int few_waves(const struct dgpu_ctx *c) { return c->n_cells <= 2 * 148 * 4 * 256; }
 
 int dgpu_create(const dgpu_sim *const *sims, int n, int device, void *stream, dgpu_ctx **out) {
@@ -795,11 +801,11 @@ int dgpu_init_state(dgpu_ctx *c, int inst) {
 
 int dctx_substep(struct dgpu_ctx *c, const TanPtrs *t, int sub) {
   /* merge beside cellprep; the sources and the phi faces beside the r faces.
-   * Up to two waves of cell blocks a launch is little longer than one thread's instruction stream, so the phi
-   * faces take a stream of their own (128 us a step for the 59,746-cell disk
-   * against 136 behind the sources, 357 against 366 for 258,078 cells); on
-   * larger contexts three kernels at once only share the SMs (the 12-disk
-   * sweep 392 against 388 ms for 80 steps) */
+   * Up to two waves of cell blocks a launch is little longer than one thread's
+   * instruction stream, so the phi faces take a stream of their own (128 us a
+   * step for the 59,746-cell disk against 136 behind the sources, 357 against
+   * 366 for 258,078 cells); on larger contexts three kernels at once mostly
+   * share the SMs (see few_waves) */
   cudaStream_t phi = few_waves(c) ? c->side2 : c->side;
   CK(cudaEventRecord(c->fork[0], c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork[0], 0));

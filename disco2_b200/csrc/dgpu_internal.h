@@ -280,7 +280,7 @@ int dgk_flux_r(const DevPtrs *d, const TanPtrs *t, int substep, void *stream);
 int dgk_update(const DevPtrs *d, const TanPtrs *t, int substep, int stop, void *stream);
 int dgk_update_stage(const DevPtrs *d, int substep, int stop, void *stream);
 /* the outflow radial boundary, its damping and cell_calc_cons on the annuli
- * it rewrites (one thread per boundary cell); after k_update, for stop >= 6 */
+ * it rewrites (eight lanes per boundary cell); after k_update, for stop >= 6 */
 int dgk_outflow(const DevPtrs *d, int stop, void *stream);
 /* 3-D disks: the z-face list (zmerge), z-face slopes, z slopes (cell_plm_rz
  * with Z_DIR), z-face fluxes, and the single-rank periodic z copy of

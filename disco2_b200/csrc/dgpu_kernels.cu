@@ -26,9 +26,10 @@
 //                                 fixed radial boundary, cell_bc_damp and
 //                                 cell_calc_cons; its first block advances the
 //                                 GravMass state
-// and, for disks with the outflow radial boundary, k_outflow per boundary cell
-// (cell_boundary_outflow_r).  k_merge runs beside k_cellprep on a second
-// stream, and k_source then k_flux_phi beside k_flux_r.
+// and, for disks with the outflow radial boundary, k_outflow, eight lanes per
+// boundary cell (cell_boundary_outflow_r).  k_merge runs beside k_cellprep on a
+// second stream, and k_source beside k_flux_r; k_flux_phi runs on a third
+// stream up to two waves of cells, behind k_source above that (dctx_substep).
 //
 // Built with -fmad=false: every expression keeps the reference's operation
 // order and rounding (double '/' and sqrt are IEEE-rounded on the GPU), so
@@ -2202,8 +2203,10 @@ static int update_grid(const DevPtrs *d, int tail) { return (d->n_cells + TBLK -
 // k_update's resident blocks of BLK threads per SM where none was tuned: the
 // built-in 4 (64 registers, spills), or 3 (80) when the cells take as many
 // waves of the 148 SMs either way: 199,428 cells 30.7 -> 28.8 us (0.233 ->
-// 0.2275 ms a step), 59,746 cells 16.4 -> 15; with a wave more 258,078 cells
-// go from 35.5 to 39.
+// 0.2275 ms a step), 59,746 cells 16.4 -> 15, 36,962 cells 0.112 -> 0.108 ms a
+// step; with a wave more 258,078 cells go from 35.5 to 39 us.  No other sizes
+// were measured.  The instances with passive scalars and the tangents exist for
+// the built-in budget alone.
 static int update_blocks_per_sm(const DevPtrs *d) {
   const long long c3 = 148LL * 3 * BLK, c4 = 148LL * 4 * BLK, n = d->n_cells;
   return (n + c3 - 1) / c3 == (n + c4 - 1) / c4 ? 3 : DGPU_MINB_UPDATE;
@@ -2214,7 +2217,6 @@ int dgk_update(const DevPtrs *d0, const TanPtrs *t, int substep, int stop, void 
   const DevPtrs *d = &h;
   if (!h.tune[DGPU_TUNE_UPDATE]) h.tune[DGPU_TUNE_UPDATE] = update_blocks_per_sm(d0);
   DGK_LAUNCH_TUNED(k_update, DGPU_TUNE_UPDATE, DGPU_MINB_UPDATE, update_grid(d, tail), TBLK, stream, substep, stop, tail,
-                  
                    (double *)NULL, (const int *)NULL);
   return (int)cudaGetLastError();
 }
