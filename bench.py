@@ -496,6 +496,7 @@ def main():
     # the roofline's kernel: the one that reads and writes the state, the only one with a share of
     # the algorithmic bytes (k_flux_r takes as long)
     dom = max((nm for nm in per_kernel if nm in STATE_SHARE), key=per_kernel.get)
+    slowest = max(per_kernel, key=per_kernel.get)
     fl = ctx.face_list(0)
     nfaces = int(len(fl["L"]))
     ncell = sim.num_cells
@@ -636,6 +637,7 @@ def main():
                          "alg_bytes": f"{s1} B (substep 1) and {s2} B (substep 2) per interior cell: "
                                       "the conserved state and phi edge the kernel reads and writes",
                          "ms_per_launch": per_kernel[dom],
+                         "slowest_kernel": slowest, "slowest_ms_per_launch": per_kernel[slowest],
                          "traffic_source": (f"copied from {traffic_src} (ncu dram__bytes_read.sum + "
                                             "dram__bytes_write.sum, one launch of the same workload); "
                                             "not measured in this run") if traffic_src else None},
