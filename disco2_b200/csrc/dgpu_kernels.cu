@@ -1451,6 +1451,11 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       const double dV = A.dv_half * dphi_n * A.dz;
       T pr[5];
       cons2prim<NV>(c, dV, r, P, pr);
+      // v_z of a cell without the v_z planes that is not finite (nan_vz); the
+      // annuli that the outflow boundary rewrites take it from obuf
+      if (NV == 4 && nan_vz(val(c[D_DDD]), val(c[D_SRR])) && !(A.kind & DGPU_AK_OUT_DST))
+        d.prim[ix(D_UZZ, QS, g)] = d.cons[ix(D_SZZ, QS, g)] =
+            (A.kind & DGPU_AK_BC_FIXED) && (A.kind & DGPU_AK_IC) ? 0.0 : NAN;
       // passive scalars: prim = cons / cons[DDD] (cell_conversion.c:98-101)
       for (int k = 0; k < np; ++k) pp[k] = cp[k] / val(c[D_DDD]);
       // the outflow boundary reads these prims before any damping; the
@@ -1458,7 +1463,8 @@ __device__ __forceinline__ void update_cell(const DevPtrs &d, const TanPtrs &tp,
       if (A.ob_off >= 0 && stop >= 6) {
 #pragma unroll
         for (int q = 0; q < 5; ++q)
-          d.obuf[(size_t)q * d.n_ob + A.ob_off + (g - A.cell_off)] = q < NV ? val(pr[q]) : 0.0;
+          d.obuf[(size_t)q * d.n_ob + A.ob_off + (g - A.cell_off)] =
+              q < NV ? val(pr[q]) : nan_vz(val(c[D_DDD]), val(c[D_SRR])) ? NAN : 0.0;
         for (int k = 0; k < np; ++k) d.obuf[(size_t)(5 + k) * d.n_ob + A.ob_off + (g - A.cell_off)] = pp[k];
       }
       const bool own = !(A.kind & DGPU_AK_OUT_DST);

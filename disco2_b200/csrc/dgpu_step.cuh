@@ -41,6 +41,13 @@ __device__ __forceinline__ void grav_t(GravT<T> &G, const InstState &S, const Di
 // plane UZZ / SZZ, a fifth of the state's traffic and about a tenth of the
 // arithmetic.  d.vz is set by the uploads; NULL: always all planes.
 __device__ __forceinline__ bool no_vz(const DevPtrs &d) { return d.vz && rd(d.vz) == 0; }
+// Its S_z is a sum of products with 0, one for each term of the other planes'
+// sums: NaN where one of those was not finite, which the sums of mass and S_r
+// show.  Left out, v_z would stay 0 in cells that are NaN otherwise.
+__device__ __forceinline__ bool nan_vz(double mass, double sr) {
+  const int top = 0x7ff00000;  // the exponent of infinities and NaN
+  return (__double2hiint(mass) & top) == top || (__double2hiint(sr) & top) == top;
+}
 
 // timestep_set_dt (timestep_set.c:16-21): the CFL minimum that k_plm_r left in
 // dtkey, clipped to Time_Max.
