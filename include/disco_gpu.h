@@ -161,7 +161,7 @@ int dgpu_autotune(dgpu_ctx *ctx, int steps, int *choice);
  * Leaves the context mid-step; reload the state before stepping again. */
 int dgpu_stage(dgpu_ctx *ctx, int phase);
 /* Per-cell intermediates after dgpu_stage (after dgpu_step_rk2: those of its
- * last substep; grad in 3-D: the r slopes): grad, gradp ([N][NUM_Q]), wiph[N],
+ * last substep, of a finite state; grad in 3-D: the r slopes): grad, gradp ([N][NUM_Q]), wiph[N],
  * RKcons[N][NUM_Q], RKtiph[N]; any pointer may be NULL. */
 int dgpu_get_stage_data(dgpu_ctx *ctx, int inst, double *grad, double *gradp, double *wiph,
                         double *rkcons, double *rktiph);
